@@ -38,6 +38,24 @@ __global__ void k_node_info(Geometry g, int* __restrict__ type, int* __restrict_
   if (ds) ds[n] = direction_state(g, x, y, z);
 }
 
+__global__ void k_solid_class(Geometry g, const unsigned char* __restrict__ mask,
+                              unsigned char* __restrict__ out) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  const int z = blockIdx.y, y = blockIdx.z;
+  if (x >= g.nx) return;
+  const long long n = x + (long long)g.nx * (z + (long long)g.nz * y);
+  int c = mask[n] ? kSolidStruct : kSolidFree;
+  static_for<1, Q>([&](auto qc) {
+    constexpr int q = decltype(qc)::value;
+    const int xs = x - cx(q), ys = y - cy(q), zs = z - cz(q);
+    if (c == kSolidFree && (unsigned)xs < (unsigned)g.nx && (unsigned)ys < (unsigned)g.ny &&
+        (unsigned)zs < (unsigned)g.nz &&
+        mask[xs + (long long)g.nx * (zs + (long long)g.nz * ys)])
+      c = kSolidNear;
+  });
+  out[n] = (unsigned char)c;
+}
+
 constexpr int kDiagThreads = 256;
 
 // per block: [mass, mom x, mom y, mom z, L1 residual, kinetic energy,
@@ -206,7 +224,12 @@ int lbm_set_solid_mask(lbm_domain* d, const unsigned char* mask) {
       d->solid = nullptr;
       return set_error(LBM_ERR_OOM, "solid mask of %lld bytes", d->N);
     }
-    CK(cudaMemcpyAsync(d->solid, mask, (size_t)d->N, cudaMemcpyHostToDevice, d->stream));
+    if ((rc = ensure_staging(d, (size_t)d->N))) return rc;
+    unsigned char* raw = (unsigned char*)d->staging;
+    CK(cudaMemcpyAsync(raw, mask, (size_t)d->N, cudaMemcpyHostToDevice, d->stream));
+    const dim3 b = block_of(d->g.nx);
+    k_solid_class<<<grid_of(d->g, b), b, 0, d->stream>>>(d->g, raw, d->solid);
+    CK(cudaGetLastError());
     d->g.solid = d->solid;
   } else {
     d->g.solid = nullptr;
