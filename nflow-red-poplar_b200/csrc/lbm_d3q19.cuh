@@ -304,8 +304,10 @@ struct MrtParams {
   // epsilon moment's difference m_2 - meq_2 that the deviations g do not
   // carry (0 for the standard weps = 3, and 0 when the populations are f)
   R e2c;
+  // factors of the fused form (populations f): -1/RefDen, wxx/RefDen, -weps,
+  // -wepsj/RefDen
+  R nr0, wr, nweps, nwj;
 };
-
 
 // ------------------------------------------------------------------ //
 // Opposite-pair form of the node arithmetic.  With s_p = f_a + f_abar and
@@ -329,6 +331,11 @@ struct PairState {
   V f0, s[9], d[9];
   V rho, jx, jy, jz;  // sum of the internal values and momentum sum c f
   V rho_full;
+  // sums of the populations f (not formed for deviations): axis pairs A =
+  // s0+s1+s2; x-z diagonals s34, x-y diagonals s56, their sum G and difference
+  // K; y-z diagonals H; all diagonals B = G + H; the third-order odd moments
+  // m16, m17 and -m18
+  V A, B, G, H, K, s34, s56, m16, m17, nm18;
 };
 
 // DEV: f holds deviations g = f - w (16-bit shifted storage)
@@ -340,6 +347,30 @@ __host__ __device__ __forceinline__ void make_pairs(const V (&f)[Q], PairState<V
     ps.s[p] = f[pair_a(p)] + f[opp(pair_a(p))];
     ps.d[p] = f[pair_a(p)] - f[opp(pair_a(p))];
   });
+  if constexpr (!DEV) {
+    // The even moments, the stress of the LES and rho read the same seven
+    // sums of s, the odd ones and j the same eight sums of d: formed once
+    // (15 + 15 additions instead of 71).
+    ps.s34 = ps.s[3] + ps.s[4];
+    ps.s56 = ps.s[5] + ps.s[6];
+    ps.G = ps.s34 + ps.s56;
+    ps.K = ps.s56 - ps.s34;
+    ps.H = ps.s[7] + ps.s[8];
+    ps.A = ps.s[0] + (ps.s[1] + ps.s[2]);
+    ps.B = ps.G + ps.H;
+    ps.rho = ps.f0 + (ps.A + ps.B);
+    ps.rho_full = ps.rho;
+    const V b = ps.d[3] - ps.d[4], t = ps.d[5] - ps.d[6];
+    ps.jx = ps.d[0] + (b + t);
+    ps.m16 = t - b;
+    const V c = ps.d[5] + ps.d[6], e = ps.d[7] + ps.d[8];
+    ps.jy = ps.d[2] + (c + e);
+    ps.m17 = e - c;
+    const V g = ps.d[8] - ps.d[7], h = ps.d[3] + ps.d[4];
+    ps.jz = (g - h) - ps.d[1];
+    ps.nm18 = g + h;
+    return;
+  }
   // rho = f0 + sum s; j_alpha = sum_p c_alpha(a_p) d_p
   V acc = ps.s[0] + ps.s[1];
   acc = acc + ps.s[2];
@@ -368,10 +399,29 @@ __host__ __device__ __forceinline__ void make_pairs(const V (&f)[Q], PairState<V
 }
 
 // Smagorinsky tau_eddy from the pair sums (same closed form as les_tau_eddy)
-template <class V>
+template <class V, bool DEV>
 __host__ __device__ __forceinline__ V les_tau_eddy_pairs(const PairState<V>& ps, V ux, V uy, V uz,
                                                          V inv_rho, V tau, V les_c) {
   const V* s = ps.s;
+  if constexpr (!DEV) {
+    const V r3 = ps.rho * bc<V>(1.0 / 3.0);
+    const V txx = (s[0] + ps.G) - fma_(ps.jx, ux, r3);
+    const V tyy = (s[2] + (ps.s56 + ps.H)) - fma_(ps.jy, uy, r3);
+    const V tzz = (s[1] + (ps.s34 + ps.H)) - fma_(ps.jz, uz, r3);
+    // the off-diagonal terms with the opposite sign: only their squares count
+    const V txy = fma_(ps.jx, uy, s[6] - s[5]);
+    const V txz = fma_(ps.jx, uz, s[3] - s[4]);
+    const V tyz = fma_(ps.jy, uz, s[7] - s[8]);
+    V off = txy * txy;
+    off = fma_(txz, txz, off);
+    off = fma_(tyz, tyz, off);
+    V qq = txx * txx;
+    qq = fma_(tyy, tyy, qq);
+    qq = fma_(tzz, tzz, qq);
+    qq = fma_(bc<V>(2), off, qq);
+    return fma_(bc<V>(0.5), vsqrt(fma_(tau, tau, (les_c * vsqrt(qq)) * inv_rho)),
+                bc<V>(-0.5) * tau);
+  }
   V pxx = s[0] + s[3];
   pxx = pxx + s[4];
   pxx = pxx + s[5];
@@ -424,7 +474,7 @@ __host__ __device__ __forceinline__ void collide_srt_pairs(const V (&f)[Q], cons
   if constexpr (DEV)
     emit(IC<0>{}, fma_(bc<V>(1.0 / 3.0) * fma_(rho, c0, ps.rho) - ps.f0, inv_tau, ps.f0));
   else
-    emit(IC<0>{}, fma_((rho * bc<V>(1.0 / 3.0)) * c0 - ps.f0, inv_tau, ps.f0));
+    emit(IC<0>{}, fma_(fma_(rho * bc<V>(1.0 / 3.0), c0, -ps.f0), inv_tau, ps.f0));
   const V wr1 = rho * bc<V>(1.0 / 18.0), wr2 = rho * bc<V>(1.0 / 36.0);
   static_for<0, 9>([&](auto pc) {
     constexpr int p = decltype(pc)::value;
@@ -458,9 +508,108 @@ __host__ __device__ __forceinline__ void collide_srt_pairs(const V (&f)[Q], cons
       const V dd = fma_(fma_(bc<V>(2), odd, -ps.d[p]), inv_tau, ps.d[p]);
       emit(IC<a>{}, bc<V>(0.5) * (ss + dd));
       emit(IC<b>{}, bc<V>(0.5) * (ss - dd));
-    } else {
+    } else if constexpr (DEV) {
       emit(IC<a>{}, fma_((even + odd) - f[a], inv_tau, f[a]));
       emit(IC<b>{}, fma_((even - odd) - f[b], inv_tau, f[b]));
+    } else {
+      const V c = fma_(bc<V>(4.5) * eu, eu, c0);
+      emit(IC<a>{}, fma_(fma_(wr, fma_(bc<V>(3), eu, c), -f[a]), inv_tau, f[a]));
+      emit(IC<b>{}, fma_(fma_(wr, fma_(bc<V>(-3), eu, c), -f[b]), inv_tau, f[b]));
+    }
+  });
+}
+
+// The same collision for populations f, with the conserved parts of the
+// moments cancelled by hand and every multiply-add explicit, so that the
+// scalar and the packed kernels round alike whatever the compiler would fuse:
+//   m1 - meq1 = 19 (B - f0 - j.j/rho0)          (M_1 f + 11 rho = 19 (B - f0))
+//   m4 - meq4 = 5/3 jx - 5 d0, likewise 6 and 8
+// About 150 additions, multiplications and fused pairs with the pair sums,
+// against 230 of the form below.
+template <bool FROM_PAIRS, class V, class R, class Emit>
+__host__ __device__ __forceinline__ void collide_mrt_fused(const V (&f)[Q], const PairState<V>& ps,
+                                                           V s_nu, const MrtParams<R>& p,
+                                                           Emit&& emit) {
+  const V* s = ps.s;
+  const V* d = ps.d;
+  const V jx = ps.jx, jy = ps.jy, jz = ps.jz;
+  const V r0 = bcast_param<V>(p.rho0_inv), nr0 = bcast_param<V>(p.nr0);
+  const V wr = bcast_param<V>(p.wr);
+  const V jxx = jx * jx, jyy = jy * jy, jzz = jz * jz;
+  const V jj = (jxx + jyy) + jzz;
+  // ---- relaxed, pre-scaled differences dm'_k = s_k (m_k - meq_k)/|row|^2 ----
+  const V e1 = bc<V>(1.19 * 19.0 / 2394.0) * fma_(jj, nr0, ps.B - ps.f0);
+  const V m2 = fma_(bc<V>(12), ps.f0, fma_(bc<V>(-4), ps.A, ps.B));
+  const V e2 = bc<V>(1.4 / 252.0) *
+               fma_(jj, bcast_param<V>(p.nwj), fma_(ps.rho, bcast_param<V>(p.nweps), m2));
+  // -rho0 meq9 = j.j - 3 jx^2, -rho0 meq11 = jz^2 - jy^2
+  const V n9 = fma_(bc<V>(-3), jxx, jj), n11 = jzz - jyy;
+  const V s12 = s[1] + s[2];
+  const V GmH = fma_(bc<V>(-2), ps.H, ps.G);
+  const V m9 = fma_(bc<V>(2), s[0], GmH - s12);
+  const V m10 = fma_(bc<V>(-4), s[0], fma_(bc<V>(2), s12, GmH));
+  const V d21 = s[2] - s[1];
+  const V m11 = d21 + ps.K;
+  const V m12 = fma_(bc<V>(-2), d21, ps.K);
+  const V e9 = (s_nu * bc<V>(1.0 / 36.0)) * fma_(n9, r0, m9);
+  const V e10 = bc<V>(1.4 / 72.0) * fma_(n9, wr, m10);
+  const V e11 = (s_nu * bc<V>(1.0 / 12.0)) * fma_(n11, r0, m11);
+  const V e12 = bc<V>(1.4 / 24.0) * fma_(n11, wr, m12);
+  const V snu4 = s_nu * bc<V>(1.0 / 4.0);
+  const V e13 = snu4 * fma_(jx * jy, nr0, s[5] - s[6]);
+  const V e14 = snu4 * fma_(jy * jz, nr0, s[8] - s[7]);
+  const V e15 = snu4 * fma_(jz * jx, nr0, s[4] - s[3]);
+  // h4 = -e4, h6 = -e6
+  const V h4 = bc<V>(1.2 / 8.0) * fma_(bc<V>(-1.0 / 3.0), jx, d[0]);
+  const V h6 = bc<V>(1.2 / 8.0) * fma_(bc<V>(-1.0 / 3.0), jy, d[2]);
+  const V e8 = bc<V>(1.2 / 8.0) * fma_(bc<V>(1.0 / 3.0), jz, d[1]);
+  const V e16 = bc<V>(1.98 / 8.0) * ps.m16;
+  const V e17 = bc<V>(1.98 / 8.0) * ps.m17;
+  const V h18 = bc<V>(1.98 / 8.0) * ps.nm18;  // -e18
+  // ---- back transform, f -= M^T dm' ----
+  emit(IC<0>{}, fma_(bc<V>(30), e1, fma_(bc<V>(-12), e2, ps.f0)));
+  const V eax = fma_(bc<V>(-11), e1, bc<V>(-4) * e2);  // rows 1,2 on axis directions
+  const V edg = fma_(bc<V>(8), e1, e2);                 // rows 1,2 on diagonals
+  const V g910 = e9 + e10;
+  const V g1112 = e11 + e12;
+  const V ax_yz = fma_(bc<V>(2), e10, eax - e9);
+  const V dx = edg + g910;
+  const V dxz = dx - g1112, dxy = dx + g1112;
+  const V dyz = fma_(bc<V>(-2), g910, edg);
+  V E[9], O[9];
+  E[0] = fma_(bc<V>(2), e9, fma_(bc<V>(-4), e10, eax));
+  O[0] = bc<V>(4) * h4;
+  E[1] = fma_(bc<V>(2), e12, ax_yz - e11);
+  O[1] = bc<V>(4) * e8;
+  E[2] = fma_(bc<V>(-2), e12, ax_yz + e11);
+  O[2] = bc<V>(4) * h6;
+  E[3] = dxz - e15;
+  E[4] = dxz + e15;
+  E[5] = dxy + e13;
+  E[6] = dxy - e13;
+  E[7] = dyz - e14;
+  E[8] = dyz + e14;
+  const V p1 = h4 + e16, q1 = e8 - h18;  // -(e4 - e16), e8 + e18
+  O[3] = p1 + q1;  // -O
+  O[4] = p1 - q1;
+  const V p2 = h4 - e16, q2 = h6 + e17;  // -(e4 + e16), -(e6 - e17)
+  O[5] = p2 + q2;  // -O
+  O[6] = p2 - q2;
+  const V q3 = e17 - h6, q4 = e8 + h18;  // e6 + e17, e8 - e18
+  O[7] = q3 - q4;
+  O[8] = q3 + q4;
+  static_for<0, 9>([&](auto qc) {
+    constexpr int q = decltype(qc)::value;
+    // pairs 3 and 5 hold -O: their a takes the difference
+    constexpr int pa = pair_a(q), a = q == 3 || q == 5 ? opp(pa) : pa, b = opp(a);
+    if constexpr (FROM_PAIRS) {
+      const V ss = fma_(bc<V>(-2), E[q], s[q]);
+      const V dd = fma_(bc<V>(-2), O[q], a == pa ? d[q] : -d[q]);
+      emit(IC<a>{}, bc<V>(0.5) * (ss + dd));
+      emit(IC<b>{}, bc<V>(0.5) * (ss - dd));
+    } else {
+      emit(IC<a>{}, f[a] - (E[q] + O[q]));
+      emit(IC<b>{}, f[b] - (E[q] - O[q]));
     }
   });
 }
@@ -477,6 +626,10 @@ template <bool FROM_PAIRS, class V, class R, bool DEV = false, class Emit>
 __host__ __device__ __forceinline__ void collide_mrt_pairs(const V (&f)[Q], const PairState<V>& ps,
                                                            V s_nu, const MrtParams<R>& p,
                                                            Emit&& emit) {
+  if constexpr (!DEV) {
+    collide_mrt_fused<FROM_PAIRS, V, R>(f, ps, s_nu, p, emit);
+    return;
+  }
   const V* s = ps.s;
   const V* d = ps.d;
   const V rho = ps.rho, jx = ps.jx, jy = ps.jy, jz = ps.jz;

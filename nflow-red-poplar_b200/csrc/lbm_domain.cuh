@@ -255,6 +255,10 @@ StepArgs<S> make_args(const lbm_domain* d, const void* src, void* dst, long long
   a.mp.wepsj = R(d->in.dWepsj);
   a.mp.wxx = R(d->in.dWXX);
   a.mp.e2c = kDev<S> ? R(3) - a.mp.weps : R(0);
+  a.mp.nr0 = -a.mp.rho0_inv;
+  a.mp.wr = a.mp.wxx * a.mp.rho0_inv;
+  a.mp.nweps = -a.mp.weps;
+  a.mp.nwj = -(a.mp.wepsj * a.mp.rho0_inv);
   // step counter of the stochastic rounding: step k reads kctr[(k-1) & 1]
   // and writes kctr[k & 1] (d->flag[2..3])
   a.kctr = (unsigned*)(d->flag + 2);

@@ -456,7 +456,7 @@ __device__ __forceinline__ void collide_node(const V (&f)[Q], const PairState<V>
   const V tau = bcast_param<V>(a.tau);
   V te = bc<V>(0);
   if constexpr (LES)
-    te = les_tau_eddy_pairs<V>(ps, ux, uy, uz, inv_rho, tau, bcast_param<V>(a.les_c));
+    te = les_tau_eddy_pairs<V, kDev<S>>(ps, ux, uy, uz, inv_rho, tau, bcast_param<V>(a.les_c));
   const V inv = vrcp(tau + te);
   if constexpr (COLL == COLL_SRT)
     collide_srt_pairs<FROM_PAIRS, V, kDev<S>>(f, ps, ux, uy, uz, inv, emit);
