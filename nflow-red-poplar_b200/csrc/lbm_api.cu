@@ -234,6 +234,8 @@ int lbm_set_solid_mask(lbm_domain* d, const unsigned char* mask) {
   } else {
     d->g.solid = nullptr;
   }
+  // the domain restarts, so its rows can change with its step kernel
+  d->g.rows = domain_rows(d);
   // the step kernel and its captured graphs depend on the geometry
   for (int i = 0; i < 2; ++i)
     if (d->chunk[i]) {

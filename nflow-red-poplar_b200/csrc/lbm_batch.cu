@@ -482,10 +482,8 @@ int issue_chunk_flat(lbm_batch* b, int steps_offered, long long* lups) {
         const lbm_domain* d = only->m->d;
         const int nb = mode == kModeAA ? p.args[0].aa_step - 1 : 0;
         kp.func = const_cast<void*>(t.single[model][mode][nb]);
-        kp.blockDim = block_of(mode == kModePaired ? d->g.px / 2 : d->g.nx);
-        kp.gridDim = dim3(((mode == kModePaired ? d->g.px / 2 : d->g.nx) + kp.blockDim.x - 1) /
-                              kp.blockDim.x,
-                          d->g.nz, d->g.ny);
+        kp.blockDim = dim3(kFlat);
+        kp.gridDim = flat_grid(d->g);
         args[0] = &p.args[0];
       } else {
         kp.func = const_cast<void*>(t.flat[model][mode]);
@@ -740,12 +738,9 @@ int lbm_batch_add(lbm_batch* b, const Inputval* pinput, const lbm_options* opt,
   if (b->free_images.empty() && (rc = grow_images(b))) return rc;
   lbm_domain* d = new lbm_domain();
   domain_prepare(d, pinput, opt);
-  // 16-bit A/B members keep the paired rows of a single domain where the
-  // paired step applies (no STRUCT nodes, nx large enough), else plain rows;
-  // AA members keep plain rows (the batched AA step is per node)
-  if (d->opt.stream_mode == LBM_STREAM_AA ||
-      (d->g.rows == kRowsPaired && !paired_kernel_applies(d->g)))
-    d->g.rows = kRowsPlain;
+  // A/B members keep the rows of a single domain; AA members plain rows (the
+  // batched AA step is per node)
+  if (d->opt.stream_mode == LBM_STREAM_AA) d->g.rows = kRowsPlain;
   d->opt.device = b->opt.device;
   d->pooled = true;
   d->stream = b->stream;

@@ -56,10 +56,6 @@ struct BatchTables {
   const unsigned char* images;   // [capacity * kImages][kArgsBytes]
 };
 
-__device__ __forceinline__ unsigned fastdiv(unsigned n, unsigned long long m) {
-  return (unsigned)__umul64hi(m, (unsigned long long)n);
-}
-
 // A warp's current domain, in shared memory (one per warp): everything the
 // tile loop needs besides the tile index, so that little stays live in
 // registers across the node step.
@@ -177,11 +173,14 @@ __global__ void __launch_bounds__(256, MINB) k_batch_step(const BatchTables* __r
       const int z = (int)(r - y * (unsigned)cur.m.nz);
       if constexpr (MODE == kModeAA)
         aa_step_node<S, COLL, LES>(a, x, (int)y, z, a.aa_step - 1,
-                                   j == 0 ? cur.m.entry0 : kAAPending);
+                                   j == 0 ? cur.m.entry0 : kAAPending,
+                                   on_face(a.g, x, (int)y, z) ? kFacesRow : kFacesNone);
       else if constexpr (MODE == kModePaired)
-        paired_word<S, COLL, LES, false>(a, x, (int)y, z);  // x: the word
+        paired_word<S, COLL, LES, false>(  // x: the word
+            a, x, (int)y, z,
+            (y == 0) | ((int)y == a.g.ny - 1) | (z == 0) | (z == a.g.nz - 1));
       else
-        step_node<S, COLL, LES>(a, x, (int)y, z);
+        step_node<S, COLL, LES>(a, x, (int)y, z, on_face(a.g, x, (int)y, z));
     }
   }
 }
@@ -232,17 +231,23 @@ __global__ void __launch_bounds__(kFlatBlock, 8)
   const StepArgs<S>& a = p.args[s];
   const FlatMeta& m = p.meta[s];
   const unsigned n = (blockIdx.x - p.cta_off[s]) * (unsigned)kFlatBlock + threadIdx.x;
-  if (n >= m.items) return;
   const unsigned r = fastdiv(n, m.mnx);
   const int x = (int)(n - r * (unsigned)m.nx);
   const unsigned y = fastdiv(r, m.mnz);
   const int z = (int)(r - y * (unsigned)m.nz);
+  // a warp that holds a node on a face (paired rows: on a y or z face) takes
+  // the face form as a whole
+  const bool row = (y == 0) | ((int)y == a.g.ny - 1) | (z == 0) | (z == a.g.nz - 1);
+  const bool rows = __any_sync(0xffffffffu, row);
+  const bool faces = MODE != kModePaired && __any_sync(0xffffffffu, (x == 0) | (x == a.g.nx - 1));
+  if (n >= m.items) return;
   if constexpr (MODE == kModeAA)
-    aa_step_node<S, COLL, LES>(a, x, (int)y, z, a.aa_step - 1, m.entry);
+    aa_step_node<S, COLL, LES>(a, x, (int)y, z, a.aa_step - 1, m.entry,
+                               rows ? kFacesRow : (faces ? kFacesX : kFacesNone));
   else if constexpr (MODE == kModePaired)
-    paired_word<S, COLL, LES, false>(a, x, (int)y, z);
+    paired_word<S, COLL, LES, false>(a, x, (int)y, z, rows);
   else
-    step_node<S, COLL, LES>(a, x, (int)y, z);
+    step_node<S, COLL, LES>(a, x, (int)y, z, rows | faces);
 }
 
 // kernel of (model, register build, mode): k[model][regs][mode];

@@ -207,6 +207,8 @@ struct StepArgs {
   unsigned long long seed;
   // batched kernel: 0 pull step, 1 AA local step, 2 AA neighbour step
   int aa_step;
+  int ri;                     // items of a row (flat_item)
+  unsigned long long mrow;
   // stochastic rounding of the 16-bit stores (paired kernel): step counter
   // pair (the step reads kctr[kpar], writes kctr[kpar ^ 1]) and seed
   unsigned* kctr;
@@ -219,6 +221,44 @@ struct StepArgs {
   // (k_aa_xface_rules)
   const float* xrule;
 };
+
+// First statement of every kernel of the step chain (launch_chained): let the
+// next kernel of the chain be scheduled as soon as every CTA of this one has
+// started, then wait until the kernel ahead is complete.  Both do nothing in
+// a plain launch.
+__device__ __forceinline__ void chain_wait() {
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+}
+
+// n / d with m = ceil(2^64 / d), exact for 32-bit n
+__device__ __forceinline__ unsigned fastdiv(unsigned n, unsigned long long m) {
+  return (unsigned)__umul64hi(m, (unsigned long long)n);
+}
+
+// The item (node, or word of paired or quad rows) of a thread in a flat grid:
+// plane y = blockIdx.y, the plane's rows one behind the other over blockIdx.x,
+// 128 to a CTA, so that few lanes are idle whatever the row length.  (One row
+// per CTA row left 37 % of the lanes of nx = 160 quad rows idle, 25 % of the CTA
+// slots at nx = 173.)  a.ri = items of a row with its padding (px nodes: a warp
+// then starts on a whole 32-byte sector; over rows of nx = 173 nodes its stores
+// split sectors and a step took 8 % longer), a.mrow = ceil(2^64 / ri).
+struct FlatItem {
+  int x, y, z;
+  bool in;        // a node (word) of the box
+  bool face_row;  // the row is on a y or z face
+};
+template <class S>
+__device__ __forceinline__ FlatItem flat_item(const StepArgs<S>& a) {
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  FlatItem i;
+  i.z = (int)fastdiv(t, a.mrow);
+  i.x = (int)t - i.z * a.ri;
+  i.y = (int)blockIdx.y;
+  i.in = i.z < a.g.nz && i.x < a.g.nx;  // words: x < px / 2 <= nx
+  i.face_row = (i.y == 0) | (i.y == a.g.ny - 1) | (i.z == 0) | (i.z == a.g.nz - 1);
+  return i;
+}
 
 // internal value of a stored population
 template <class S>
@@ -414,35 +454,73 @@ __device__ __forceinline__ void pull_struct(RealOf<S> (&f)[Q], const StepArgs<S>
   }
 }
 
+// Boundary rules of a node whose populations with a donor outside the box hold
+// the node's own f*_{opp q}.  Only two kinds of node change the value (a fixed
+// wall keeps it): the cavity's lid (y = ny - 1 off its edges, the five
+// populations with c_y = -1), and the inlet and outlet of rows off the y and z
+// faces (x = 0, c_x = +1; x = nx - 1, c_x = -1).
+template <class S>
+__device__ __forceinline__ void face_rules(RealOf<S> (&f)[Q], const StepArgs<S>& a, int x, int y,
+                                           int z, bool face_row) {
+  const bool xlo = x == 0, xhi = x == a.g.nx - 1;
+  if (a.g.casetype == CAVITY) {
+    if (y == a.g.ny - 1 && z > 0 && z < a.g.nz - 1 && !xlo && !xhi) {
+      static_for<0, Q>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        if constexpr (cy(q) == -1) f[q] = boundary_value<S, q>(a, NODE_MOVINGWALL, f[q], y, z);
+      });
+    }
+  } else if (!face_row) {
+    if (xlo) {
+      static_for<0, Q>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        if constexpr (cx(q) == 1) f[q] = boundary_value<S, q>(a, NODE_INLET, f[q], y, z);
+      });
+    }
+    if (xhi) {
+      static_for<0, Q>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        if constexpr (cx(q) == -1) f[q] = boundary_value<S, q>(a, NODE_OUTLET, f[q], y, z);
+      });
+    }
+  }
+}
+
 // Steps 1-2: the post-stream, post-boundary populations f_k at (x,y,z);
-// cell is the node's in-plane index.
+// cell is the node's in-plane index.  A node off the faces reads its donors; the
+// others choose donor or own population per lane by address (the test of the
+// donor's row is uniform along the row) and then take the rules.  faces: take
+// that form, true at least for nodes on a face; the kernels pass it to a whole
+// warp that holds one, so that the warp does not run both.  (When each lane
+// took its own form, with the rules of every node type inlined 18 times, a
+// 16^3 FP32 step took 3.8 us, 64^3 9.3 us and 96^3 27.3 us; now 2.1, 6.7 and 22.4.)
 template <class S, class Addr>
 __device__ __forceinline__ void pull(RealOf<S> (&f)[Q], const StepArgs<S>& a, const Addr& ad, int x,
-                                     int y, int z) {
-  const bool edge = (x == 0) | (x == a.g.nx - 1) | (y == 0) | (y == a.g.ny - 1) | (z == 0) |
-                    (z == a.g.nz - 1);
+                                     int y, int z, bool faces) {
   if (has_struct(a.g) && struct_class(a.g, x, y, z) != kSolidFree) {
     pull_struct<S>(f, a, ad, x, y, z);
-  } else if (!edge) {
+  } else if (!faces) {
     static_for<0, Q>([&](auto qc) {
       constexpr int q = decltype(qc)::value;
       f[q] = ld(ad.donor(q), q, ad.inv_scale());
     });
   } else {
-    const int t = node_type(a.g, x, y, z);
+    const bool xlo = x == 0, xhi = x == a.g.nx - 1;
     static_for<0, Q>([&](auto qc) {
       constexpr int q = decltype(qc)::value;
-      const int xs = x - cx(q), ys = y - cy(q), zs = z - cz(q);
-      const bool inside = (unsigned)xs < (unsigned)a.g.nx && (unsigned)ys < (unsigned)a.g.ny &&
-                          (unsigned)zs < (unsigned)a.g.nz;
-      if (inside) {
-        f[q] = ld(ad.donor(q), q, ad.inv_scale());
-      } else {
-        const RealOf<S> fo = ld(ad.own(opp(q)), opp(q), ad.inv_scale());
-        f[q] = boundary_value<S, q>(a, t, fo, y, z);
-      }
+      const bool row_out = (unsigned)(y - cy(q)) >= (unsigned)a.g.ny ||
+                           (unsigned)(z - cz(q)) >= (unsigned)a.g.nz;
+      const bool out = row_out || (cx(q) == 1 && xlo) || (cx(q) == -1 && xhi);
+      f[q] = ld(out ? ad.own(opp(q)) : ad.donor(q), q, ad.inv_scale());
     });
+    face_rules<S>(f, a, x, y, z,
+                  (y == 0) | (y == a.g.ny - 1) | (z == 0) | (z == a.g.nz - 1));
   }
+}
+
+// the node lies on a face of the box
+__device__ __forceinline__ bool on_face(const Geometry& g, int x, int y, int z) {
+  return (x == 0) | (x == g.nx - 1) | (y == 0) | (y == g.ny - 1) | (z == 0) | (z == g.nz - 1);
 }
 
 enum { COLL_SRT = 0, COLL_MRT = 1 };
@@ -586,13 +664,13 @@ __device__ __forceinline__ void finish_node(const RealOf<S> (&f)[Q], const StepA
 // arguments are held differs, not the arithmetic).
 template <class S, int COLL, bool LES, bool SR = false, class Addr>
 __device__ __forceinline__ void step_node_at(const StepArgs<S>& a, const Addr& ad, int x, int y,
-                                             int z) {
+                                             int z, bool faces) {
   using R = RealOf<S>;
   // STRUCT nodes are never streamed, collided or measured (kernel.cu:294,
   // 323, 362, 464, 495, 1105)
   if (has_struct(a.g) && struct_class(a.g, x, y, z) == kSolidStruct) return;
   R f[Q];
-  pull<S>(f, a, ad, x, y, z);
+  pull<S>(f, a, ad, x, y, z, faces);
   finish_node<S, COLL, LES, SR>(f, a, ad, x, y, z);
 }
 
@@ -606,18 +684,20 @@ __device__ __forceinline__ void bump_step_counter(const StepArgs<S>& a) {
   }
 }
 template <class S, int COLL, bool LES>
-__device__ __forceinline__ void step_node(const StepArgs<S>& a, int x, int y, int z) {
-  step_node_at<S, COLL, LES>(a, PlaneAddr<S>(a, x + a.g.px * (z + a.g.nz * y)), x, y, z);
+__device__ __forceinline__ void step_node(const StepArgs<S>& a, int x, int y, int z, bool faces) {
+  step_node_at<S, COLL, LES>(a, PlaneAddr<S>(a, x + a.g.px * (z + a.g.nz * y)), x, y, z, faces);
 }
 
-// The fused step.  grid = (ceil(nx/blockDim.x), nz, ny), one thread per node.
+// The fused step.  grid = flat_grid, one thread per node.
 template <class S, int COLL, bool LES, bool SR = false>
 __global__ void __launch_bounds__(128) k_step(const __grid_constant__ StepArgs<S> a) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int z = blockIdx.y, y = blockIdx.z;
+  chain_wait();
   bump_step_counter<SR>(a);
-  if (x >= a.g.nx) return;
-  step_node_at<S, COLL, LES, SR>(a, PlaneAddr<S>(a, x + a.g.px * (z + a.g.nz * y)), x, y, z);
+  const FlatItem i = flat_item(a);
+  const bool faces = __any_sync(0xffffffffu, i.face_row | (i.x == 0) | (i.x == a.g.nx - 1));
+  if (!i.in) return;
+  step_node_at<S, COLL, LES, SR>(a, PlaneAddr<S>(a, i.x + a.g.px * (i.z + a.g.nz * i.y)), i.x, i.y,
+                                 i.z, faces);
 }
 
 // ------------------------------------------------------------------ //
@@ -818,16 +898,9 @@ __device__ __forceinline__ RealOf<S> aa_wall(const StepArgs<S>& a, int t, RealOf
 template <class S>
 __device__ __forceinline__ void aa_open_face_rules(RealOf<S> (&f)[Q], const StepArgs<S>& a, int x,
                                                    int y, int z) {
-  if (a.g.casetype != CHANNEL) return;
-  const int t = node_type(a.g, x, y, z);
-  if (t != NODE_INLET && t != NODE_OUTLET) return;
-  static_for<0, Q>([&](auto qc) {
-    constexpr int q = decltype(qc)::value;
-    const int xs = x - cx(q), ys = y - cy(q), zs = z - cz(q);
-    const bool inside = (unsigned)xs < (unsigned)a.g.nx && (unsigned)ys < (unsigned)a.g.ny &&
-                        (unsigned)zs < (unsigned)a.g.nz;
-    if (!inside) f[q] = boundary_value<S, q>(a, t, f[q], y, z);
-  });
+  if (a.g.casetype == CHANNEL)
+    face_rules<S>(f, a, x, y, z,
+                  (y == 0) | (y == a.g.ny - 1) | (z == 0) | (z == a.g.nz - 1));
 }
 
 // Slot addresses of an AA step, set per step in the kernel parameters so
@@ -844,35 +917,37 @@ struct AADst {
   __device__ __forceinline__ float scale() const { return a.scale; }
 };
 
-// The neighbour step of a node in a row that is not on a y or z face, for
-// the warps that hold an x face of such rows.  Only the populations whose
-// donor x - c_q or destination x + c_q leaves the box at x = 0 or x = nx-1
-// differ from the interior form, and only in their slot: a donor outside is
-// the node's own slot (x, q) (the wall rule of the node applied to it, which
-// for the cavity's fixed walls is the value itself), a destination outside
-// is the node's own slot (x, opp q) (the plain f*_q: x faces are fixed
-// walls, inlets or outlets, whose rules are applied when the natural slot
-// is read).  The slot is chosen per lane, so the warp does not diverge.
-template <class S, int COLL, bool LES>
-__device__ __forceinline__ void aa_neighbor_xface_node(const StepArgs<S>& a, int x, int y, int z,
-                                                       int cell) {
+// The neighbour step of a node whose donors or destinations may lie outside
+// the box.  Each such slot is one of the node's own: the donor's is (x, q),
+// to which the node's rule applies, the destination's is (x, opp q), which takes
+// the wall value (the lid's term; the plain f*_q at inlets and outlets, whose
+// rules are applied when the natural slot is read).  The slot is chosen per
+// lane by address, so only the rules diverge.  ROWS: the row may lie on a y or
+// z face; without it only x = 0 and x = nx - 1 are looked at, which is what
+// most of the warps need that come here.  (With one form for both the 256^3
+// FP32 neighbour step took 516 us, with two 430 us.)
+template <class S, int COLL, bool LES, bool ROWS>
+__device__ __forceinline__ void aa_neighbor_face_node(const StepArgs<S>& a, int x, int y, int z,
+                                                      int cell) {
   using R = RealOf<S>;
   const bool xlo = x == 0, xhi = x == a.g.nx - 1;
+  auto row_in = [&](int dy, int dz) {
+    if constexpr (!ROWS) return true;
+    return (unsigned)(y + dy) < (unsigned)a.g.ny && (unsigned)(z + dz) < (unsigned)a.g.nz;
+  };
   R f[Q];
   static_for<0, Q>([&](auto qc) {
     constexpr int q = decltype(qc)::value;
-    const bool out = (cx(q) == 1 && xlo) || (cx(q) == -1 && xhi);
+    const bool out = !row_in(-cy(q), -cz(q)) || (cx(q) == 1 && xlo) || (cx(q) == -1 && xhi);
     f[q] = ld((out ? a.srcq[q] : a.srcd[q]) + cell, q, a.inv_scale);
   });
-  if (a.g.casetype != CAVITY && (xlo || xhi)) {
-    // inlet / outlet rules on the donors outside (the cavity's walls keep
-    // the value)
-    const int t = node_type(a.g, x, y, z);
-    static_for<0, Q>([&](auto qc) {
-      constexpr int q = decltype(qc)::value;
-      if ((cx(q) == 1 && xlo) || (cx(q) == -1 && xhi))
-        f[q] = boundary_value<S, q>(a, t, f[q], y, z);
-    });
+  [[maybe_unused]] bool lid = false;
+  if constexpr (ROWS) {
+    face_rules<S>(f, a, x, y, z,
+                  (y == 0) | (y == a.g.ny - 1) | (z == 0) | (z == a.g.nz - 1));
+    lid = a.g.casetype == CAVITY && y == a.g.ny - 1 && z > 0 && z < a.g.nz - 1 && !xlo && !xhi;
+  } else if (a.g.casetype != CAVITY) {
+    face_rules<S>(f, a, x, y, z, false);
   }
   PairState<R> ps;
   make_pairs<R, kDev<S>>(f, ps);
@@ -881,7 +956,9 @@ __device__ __forceinline__ void aa_neighbor_xface_node(const StepArgs<S>& a, int
   write_macro<S>(a, x, y, z, ps.rho_full, ux, uy, uz);
   collide_node<S, COLL, LES, kFromPairs<S>, R>(f, ps, ux, uy, uz, inv_rho, a, [&](auto qc, R v) {
     constexpr int q = decltype(qc)::value;
-    const bool out = (cx(q) == -1 && xlo) || (cx(q) == 1 && xhi);
+    const bool out = !row_in(cy(q), cz(q)) || (cx(q) == -1 && xlo) || (cx(q) == 1 && xhi);
+    if constexpr (ROWS && cy(q) == 1)
+      if (lid) v = aa_wall<S>(a, NODE_MOVINGWALL, v, q);
     StoreTraits<S>::store(out ? a.dst + (opp(q) * a.qs + cell) : a.dstq[q] + cell, v, a.scale);
   });
 }
@@ -894,103 +971,74 @@ __device__ __forceinline__ void aa_neighbor_xface_node(const StepArgs<S>& a, int
 // the pull form; kAAComplete, the slots hold arF (after an import).
 // a.src = a.dst = the lattice.
 enum { kAAPending = 0, kAAFromInit = 1, kAAComplete = 2 };
+enum { kFacesNone = 0, kFacesX = 1, kFacesRow = 2 };
 
-//
-// warp_row: the caller maps the lanes of a warp to the x-consecutive nodes
-// x - lane .. x - lane + 31 of one row (the single-domain kernel), so that
-// "this warp holds an x face" is known to every lane without a vote and a
-// warp of an interior row that holds one takes the x-face form as a whole.
-// Otherwise (the batched kernel, whose warps may span rows) each lane
-// decides for itself.
-template <class S, int COLL, bool LES, bool WARP_ROW = false>
+// faces: the form of the neighbour step: kFacesNone, kFacesX (nodes at x = 0 or
+// x = nx - 1 among the warp's) or kFacesRow (nodes on a y or z face).
+template <class S, int COLL, bool LES>
 __device__ __forceinline__ void aa_step_node(const StepArgs<S>& a, int x, int y, int z,
-                                             int neighbor, int entry) {
+                                             int neighbor, int entry, int faces) {
   using R = RealOf<S>;
-  // quad rows (16-bit storage) reach this per-node step only as a local
-  // step, whose slots are all at the node
-  const int cell = kDev<S> ? cell_of(a.g, x, y, z) : x + a.g.px * (z + a.g.nz * y);
-  const bool face_row = (y == 0) | (y == a.g.ny - 1) | (z == 0) | (z == a.g.nz - 1);
-  const bool xface = (x == 0) | (x == a.g.nx - 1);
-  const bool edge = face_row | xface;
-  bool xsel = xface;
-  if constexpr (WARP_ROW) {
-    const int x0 = x - (int)(threadIdx.x & 31u);  // the warp's first node
-    xsel = x0 == 0 || (unsigned)(a.g.nx - 1 - x0) < 32u;
+  // paired and quad rows reach this per-node step only as a local step,
+  // whose slots are all at the node
+  const int cell = neighbor ? x + a.g.px * (z + a.g.nz * y) : cell_of(a.g, x, y, z);
+  if (neighbor && faces != kFacesNone) {
+    if (faces == kFacesX)
+      aa_neighbor_face_node<S, COLL, LES, false>(a, x, y, z, cell);
+    else
+      aa_neighbor_face_node<S, COLL, LES, true>(a, x, y, z, cell);
+    return;
   }
   R f[Q];
-  if (neighbor && !face_row && xsel) {
-    aa_neighbor_xface_node<S, COLL, LES>(a, x, y, z, cell);
-    return;
-  }
-  if (!neighbor || !edge) {
-    static_for<0, Q>([&](auto qc) {
-      constexpr int q = decltype(qc)::value;
-      f[q] = ld(a.srcd[q] + cell, q, a.inv_scale);
-    });
-    if (!neighbor && edge && entry == kAAPending) aa_open_face_rules<S>(f, a, x, y, z);
-    const AADst<S> ad{a, cell};
-    if (entry != kAAFromInit) {
-      finish_node<S, COLL, LES>(f, a, ad, x, y, z);
-    } else {
-      const int t = node_type(a.g, x, y, z);
-      const InitState is = initial_state(a.g, a.init_kind, a.seed, a.noise_amp, (float)a.rho0,
-                                         (float)a.ulx, (float)a.uly, (float)a.ulz, a.inlet_u, x,
-                                         y, z, t);
-      const R rd = R(is.den), ux = R(is.ux), uy = R(is.uy), uz = R(is.uz);
-      write_macro<S>(a, x, y, z, rd, ux, uy, uz);
-      PairState<R> ps;
-      make_pairs<R, kDev<S>>(f, ps);
-      ps.rho = kDev<S> ? rd - R(1) : rd;
-      ps.rho_full = rd;
-      ps.jx = mul_rn(rd, ux);
-      ps.jy = mul_rn(rd, uy);
-      ps.jz = mul_rn(rd, uz);
-      collide_node<S, COLL, LES, kFromPairs<S>, R>(f, ps, ux, uy, uz, vrcp(rd), a, [&](int q, R v) {
-        StoreTraits<S>::store(ad.out(q), v, ad.scale());
-      });
-    }
-    return;
-  }
-  // neighbour step at a box face: slots outside the box are the node's own
-  const int t = node_type(a.g, x, y, z);
   static_for<0, Q>([&](auto qc) {
     constexpr int q = decltype(qc)::value;
-    const int xs = x - cx(q), ys = y - cy(q), zs = z - cz(q);
-    const bool inside = (unsigned)xs < (unsigned)a.g.nx && (unsigned)ys < (unsigned)a.g.ny &&
-                        (unsigned)zs < (unsigned)a.g.nz;
-    if (inside) {
-      f[q] = ld(a.srcd[q] + cell, q, a.inv_scale);
-    } else {
-      const RealOf<S> fo = ld(a.srcq[q] + cell, q, a.inv_scale);  // own f*_{opp q}
-      f[q] = boundary_value<S, q>(a, t, fo, y, z);
-    }
+    f[q] = ld(a.srcd[q] + cell, q, a.inv_scale);
   });
+  const AADst<S> ad{a, cell};
+  if (neighbor || entry != kAAFromInit) {
+    if (!neighbor && entry == kAAPending && ((x == 0) | (x == a.g.nx - 1)))
+      aa_open_face_rules<S>(f, a, x, y, z);
+    finish_node<S, COLL, LES>(f, a, ad, x, y, z);
+    return;
+  }
+  // the first step after the initial state
+  const int t = node_type(a.g, x, y, z);
+  const InitState is = initial_state(a.g, a.init_kind, a.seed, a.noise_amp, (float)a.rho0,
+                                     (float)a.ulx, (float)a.uly, (float)a.ulz, a.inlet_u, x, y, z,
+                                     t);
+  const R rd = R(is.den), ux = R(is.ux), uy = R(is.uy), uz = R(is.uz);
+  write_macro<S>(a, x, y, z, rd, ux, uy, uz);
   PairState<R> ps;
   make_pairs<R, kDev<S>>(f, ps);
-  R ux, uy, uz;
-  const R inv_rho = velocity<R>(ps, ux, uy, uz);
-  write_macro<S>(a, x, y, z, ps.rho_full, ux, uy, uz);
-  collide_node<S, COLL, LES, kFromPairs<S>, R>(f, ps, ux, uy, uz, inv_rho, a, [&](int q, R v) {
-    const int xt = x + cx(q), yt = y + cy(q), zt = z + cz(q);
-    const bool inside = (unsigned)xt < (unsigned)a.g.nx && (unsigned)yt < (unsigned)a.g.ny &&
-                        (unsigned)zt < (unsigned)a.g.nz;
-    if (inside)
-      StoreTraits<S>::store(a.dstq[q] + cell, v, a.scale);
-    else
-      StoreTraits<S>::store(a.dst + (opp(q) * a.qs + cell), aa_wall<S>(a, t, v, q), a.scale);
+  ps.rho = kDev<S> ? rd - R(1) : rd;
+  ps.rho_full = rd;
+  ps.jx = mul_rn(rd, ux);
+  ps.jy = mul_rn(rd, uy);
+  ps.jz = mul_rn(rd, uz);
+  collide_node<S, COLL, LES, kFromPairs<S>, R>(f, ps, ux, uy, uz, vrcp(rd), a, [&](int q, R v) {
+    StoreTraits<S>::store(ad.out(q), v, ad.scale());
   });
 }
 
 // One kernel per step kind (NB = neighbor): the local step, which has no
 // box-face logic besides the open-face rules, fits 56 registers (9 CTAs of
-// 128 per SM) without spills; the neighbour step keeps 64.
+// 128 per SM) without spills; the neighbour step takes 72 (7 CTAs), as with
+// 64 it spills 60 bytes: 256^3 FP32 412 us a step (mean of both kinds) against
+// 422, 512x128x128 204 against 213.
 template <class S, int COLL, bool LES, int NB>
-__global__ void __launch_bounds__(128, NB ? 8 : 9)
+__global__ void __launch_bounds__(128, NB ? 7 : 9)
     k_aa_step(const __grid_constant__ StepArgs<S> a, int entry) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int z = blockIdx.y, y = blockIdx.z;
-  if (x >= a.g.nx) return;
-  aa_step_node<S, COLL, LES, true>(a, x, y, z, NB, entry);
+  chain_wait();
+  const FlatItem i = flat_item(a);
+  int faces = kFacesNone;
+  if constexpr (NB) {
+    if (__any_sync(0xffffffffu, i.face_row))
+      faces = kFacesRow;
+    else if (__any_sync(0xffffffffu, (i.x == 0) | (i.x == a.g.nx - 1)))
+      faces = kFacesX;
+  }
+  if (!i.in) return;
+  aa_step_node<S, COLL, LES>(a, i.x, i.y, i.z, NB, entry, faces);
 }
 
 // rho and u of arF in the current AA layout, written through a.den_out /
@@ -1002,6 +1050,7 @@ enum { kAANaturalComplete = 0, kAASwapped = 1, kAANaturalPending = 2 };
 template <class S>
 __global__ void __launch_bounds__(128) k_aa_macro(const __grid_constant__ StepArgs<S> a,
                                                   int layout) {
+  chain_wait();
   using R = RealOf<S>;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int z = blockIdx.y, y = blockIdx.z;
@@ -1055,9 +1104,9 @@ __global__ void __launch_bounds__(128)
   } else if (mode == kExportAASwapped) {
     aa_pull_swapped<S>(f, a, x, y, z, (int)cell);
   } else if (a.g.rows != kRowsPlain) {
-    pull<S>(f, a, RowAddr<S>(a, x, y, z), x, y, z);
+    pull<S>(f, a, RowAddr<S>(a, x, y, z), x, y, z, on_face(a.g, x, y, z));
   } else {
-    pull<S>(f, a, PlaneAddr<S>(a, (int)cell), x, y, z);
+    pull<S>(f, a, PlaneAddr<S>(a, (int)cell), x, y, z, on_face(a.g, x, y, z));
   }
   long long node;
   if (padded)
@@ -1143,9 +1192,9 @@ __global__ void __launch_bounds__(64, LBM_PACKED_MIN_BLOCKS) k_step2(const __gri
     });
   } else {
     float fa[Q], fb[Q];
-    pull<S>(fa, a, PlaneAddr<S>(a, cell), x0, y, z);
+    pull<S>(fa, a, PlaneAddr<S>(a, cell), x0, y, z, true);
     if (two) {
-      pull<S>(fb, a, PlaneAddr<S>(a, cell + 1), x0 + 1, y, z);
+      pull<S>(fb, a, PlaneAddr<S>(a, cell + 1), x0 + 1, y, z, true);
     } else {
       static_for<0, Q>([&](auto qc) { fb[decltype(qc)::value] = fa[decltype(qc)::value]; });
     }
@@ -1199,7 +1248,7 @@ __global__ void __launch_bounds__(64, LBM_PACKED_MIN_BLOCKS) k_step2(const __gri
 // last node (x >= nx when nx < px) compute on padding slots, which no real
 // node reads and nothing exports.  The node types and rules are those of
 // the per-node path, which steps the geometries with STRUCT nodes
-// (k_step_rows); the 16-bit units are built without multiply-add
+// over plain rows; the FP32 and 16-bit units are built without multiply-add
 // contraction and both paths rebuild f* from the pair sums, so a node gets
 // the same bits from either.
 // ------------------------------------------------------------------ //
@@ -1251,8 +1300,8 @@ __device__ __forceinline__ uint32_t pack_pair_sr<__nv_bfloat16>(F2 v, float scal
   return d;
 }
 
-// the paired step kernel applies to the domain (else: k_step_rows); nx >=
-// 11 keeps both x faces out of each other's words and every hi lane's x + 1
+// the paired step kernel applies to the domain (else: plain rows); nx >= 11
+// keeps both x faces out of each other's words and every hi lane's x + 1
 // donor of a real node inside the row
 __host__ __device__ __forceinline__ bool paired_kernel_applies(const Geometry& g) {
   return !has_struct(g) && (g.px >> 1) <= g.nx - 2;
@@ -1266,76 +1315,106 @@ __host__ __device__ __forceinline__ bool paired_kernel_applies(const Geometry& g
 #define LBM_PAIRED_THREADS_PER_SM 1024
 #endif
 
-// grid = (ceil(H / b), nz, ny), b = H rounded up to a multiple of 32 and
-// at most 128 threads, one word (two nodes) per thread; a.srcd[q] = plane q
-// minus the donor offset 2 c_x + px (c_z + nz c_y)
+// grid = flat_grid, one word (two nodes) per thread; a.srcd[q] = plane q minus
+// the donor offset 2 c_x + px (c_z + nz c_y)
 #ifndef LBM_PAIRED_SR_THREADS_PER_SM
 #define LBM_PAIRED_SR_THREADS_PER_SM 768
 #endif
 // One word w (0 <= w < px/2) of row (y, z): the step of its two nodes
-// (shared by the single-domain and batched kernels).
+// (shared by the single-domain and batched kernels).  faces: some lane of the
+// caller's warp is in a row on a y or z face (that row at least must pass it).
 template <class S, int COLL, bool LES, bool SR>
-__device__ __forceinline__ void paired_word(const StepArgs<S>& a, int w, int y, int z) {
+__device__ __forceinline__ void paired_word(const StepArgs<S>& a, int w, int y, int z, bool faces) {
   static_assert(kDev<S>, "paired rows are a 16-bit layout");
   const int H = a.g.px >> 1;
   const int xh = w + H;                             // node of the hi lane
   const int e = 2 * w + a.g.px * (z + a.g.nz * y);  // the pair's word (lo slot)
   const bool face_row = y == 0 || y == a.g.ny - 1 || z == 0 || z == a.g.nz - 1;
+  const bool xlo = w == 0, xhi = xh == a.g.nx - 1;
+  auto ldw = [&](const S* p) {
+    return unpack_pair<S>(*reinterpret_cast<const uint32_t*>(p), a.inv_scale);
+  };
+  auto row_in = [&](int q) {
+    return (unsigned)(y - cy(q)) < (unsigned)a.g.ny && (unsigned)(z - cz(q)) < (unsigned)a.g.nz;
+  };
   F2 f[Q];
-  if (!face_row) {
+  if (!faces) {
     static_for<0, Q>([&](auto qc) {
       constexpr int q = decltype(qc)::value;
-      f[q] = unpack_pair<S>(*reinterpret_cast<const uint32_t*>(a.srcd[q] + e), a.inv_scale);
+      f[q] = ldw(a.srcd[q] + e);
     });
   } else {
-    const int t_lo = node_type(a.g, w, y, z);
-    const int t_hi = xh < a.g.nx ? node_type(a.g, xh, y, z) : NODE_FLUID;
     static_for<0, Q>([&](auto qc) {
       constexpr int q = decltype(qc)::value;
-      const bool inside = (unsigned)(y - cy(q)) < (unsigned)a.g.ny &&
-                          (unsigned)(z - cz(q)) < (unsigned)a.g.nz;
-      if (inside) {
-        f[q] = unpack_pair<S>(*reinterpret_cast<const uint32_t*>(a.srcd[q] + e), a.inv_scale);
-      } else {
-        const F2 fo = unpack_pair<S>(*reinterpret_cast<const uint32_t*>(a.srcq[opp(q)] + e),
-                                     a.inv_scale);
-        f[q] = mk2(boundary_value<S, q>(a, t_lo, fo.v.x, y, z),
-                   boundary_value<S, q>(a, t_hi, fo.v.y, y, z));
+      f[q] = ldw((row_in(q) ? a.srcd[q] : a.srcq[opp(q)]) + e);
+    });
+  }
+  // the seam and the x faces (see above): the word across the seam, and the
+  // node's own word where its donor is outside.  All ten words are fetched
+  // before the first is used; where the donor's row is outside f holds the
+  // own word already.
+  const int e0 = e - 2 * w;  // row start
+  if (xlo) {
+    F2 own[Q], across[Q];
+    static_for<0, Q>([&](auto qc) {
+      constexpr int q = decltype(qc)::value;
+      if constexpr (cx(q) == 1) {
+        own[q] = ldw(a.srcq[opp(q)] + e);
+        across[q] = ldw(row_in(q) ? a.srcd[q] + (e0 + a.g.px) : a.srcq[opp(q)] + e);
+      }
+    });
+    static_for<0, Q>([&](auto qc) {
+      constexpr int q = decltype(qc)::value;
+      if constexpr (cx(q) == 1) {
+        f[q].v.x = own[q].v.x;
+        if (row_in(q)) f[q].v.y = across[q].v.x;  // x = H takes node H - 1
       }
     });
   }
-  if (w == 0 || w == H - 1 || xh == a.g.nx - 1) {
-    // the seam and the x faces (see above), lane by lane
-    const int e0 = e - 2 * w;  // row start
-    const int t_lo = node_type(a.g, w, y, z);
-    const int t_hi = xh < a.g.nx ? node_type(a.g, xh, y, z) : NODE_FLUID;
+  if (xhi || w == H - 1) {
+    F2 own[Q], across[Q];
     static_for<0, Q>([&](auto qc) {
       constexpr int q = decltype(qc)::value;
-      if constexpr (cx(q) != 0) {
-        const bool inside = !face_row || ((unsigned)(y - cy(q)) < (unsigned)a.g.ny &&
-                                          (unsigned)(z - cz(q)) < (unsigned)a.g.nz);
-        if (inside) {
-          const int ws = cx(q) == 1 ? H - 1 : 0;  // the word across the seam
-          if ((cx(q) == 1 && w == 0) || (cx(q) == -1 && w == H - 1)) {
-            const uint32_t sw =
-                *reinterpret_cast<const uint32_t*>(a.srcd[q] + (e0 + 2 * ws + 2 * cx(q)));
-            const F2 v = unpack_pair<S>(sw, a.inv_scale);
-            if (cx(q) == 1)
-              f[q].v.y = v.v.x;  // x = H takes node H - 1
-            else
-              f[q].v.x = v.v.y;  // x = H - 1 takes node H
-          }
-          const bool lo_out = cx(q) == 1 && w == 0;
-          const bool hi_out = cx(q) == -1 && xh == a.g.nx - 1;
-          if (lo_out || hi_out) {
-            const F2 fo = unpack_pair<S>(*reinterpret_cast<const uint32_t*>(a.srcq[opp(q)] + e),
-                                         a.inv_scale);
-            if (lo_out) f[q].v.x = boundary_value<S, q>(a, t_lo, fo.v.x, y, z);
-            if (hi_out) f[q].v.y = boundary_value<S, q>(a, t_hi, fo.v.y, y, z);
-          }
-        }
+      if constexpr (cx(q) == -1) {
+        own[q] = ldw(a.srcq[opp(q)] + e);
+        across[q] = ldw(row_in(q) ? a.srcd[q] + (e0 - 2) : a.srcq[opp(q)] + e);
       }
     });
+    static_for<0, Q>([&](auto qc) {
+      constexpr int q = decltype(qc)::value;
+      if constexpr (cx(q) == -1) {
+        if (w == H - 1 && row_in(q)) f[q].v.x = across[q].v.y;  // x = H - 1 takes node H
+        if (xhi) f[q].v.y = own[q].v.y;
+      }
+    });
+  }
+  // the rules that change the value, as in face_rules
+  if (a.g.casetype == CAVITY) {
+    if (y == a.g.ny - 1 && z > 0 && z < a.g.nz - 1) {
+      static_for<0, Q>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        if constexpr (cy(q) == -1) {
+          const F2 fo = f[q];
+          if (!xlo) f[q].v.x = boundary_value<S, q>(a, NODE_MOVINGWALL, fo.v.x, y, z);
+          if (!xhi) f[q].v.y = boundary_value<S, q>(a, NODE_MOVINGWALL, fo.v.y, y, z);
+        }
+      });
+    }
+  } else if (!face_row) {
+    if (xlo) {
+      static_for<0, Q>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        if constexpr (cx(q) == 1)
+          f[q].v.x = boundary_value<S, q>(a, NODE_INLET, f[q].v.x, y, z);
+      });
+    }
+    if (xhi) {
+      static_for<0, Q>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        if constexpr (cx(q) == -1)
+          f[q].v.y = boundary_value<S, q>(a, NODE_OUTLET, f[q].v.y, y, z);
+      });
+    }
   }
   PairState<F2> ps;
   make_pairs<F2, true>(f, ps);
@@ -1350,9 +1429,6 @@ __device__ __forceinline__ void paired_word(const StepArgs<S>& a, int w, int y, 
       *reinterpret_cast<uint32_t*>(a.dstq[q] + e) = pack_pair<S>(v, a.scale);
     });
   } else {
-    // the step number: this step reads kctr[kpar] and leaves its successor
-    // in kctr[kpar ^ 1] for the next step
-    bump_step_counter<SR>(a);
     const uint32_t h = sr_hash((uint32_t)(e >> 1), a.kctr[a.kpar], a.sr_seed);
     collide_node<S, COLL, LES, true, F2>(f, ps, ux, uy, uz, inv_rho, a, [&](auto qc, F2 v) {
       constexpr int q = decltype(qc)::value;
@@ -1365,21 +1441,12 @@ template <class S, int COLL, bool LES, bool SR>
 __global__ void __launch_bounds__(128, (SR ? LBM_PAIRED_SR_THREADS_PER_SM
                                            : LBM_PAIRED_THREADS_PER_SM) / 128)
     k_step_paired(const __grid_constant__ StepArgs<S> a) {
-  const int w = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int z = blockIdx.y, y = blockIdx.z;
-  if (w >= (a.g.px >> 1)) return;
-  paired_word<S, COLL, LES, SR>(a, w, y, z);
-}
-
-// Paired domains the paired kernel does not apply to (STRUCT nodes, nx <
-// 11): the per-node step over paired rows.  grid = (ceil(nx/128), nz, ny).
-template <class S, int COLL, bool LES, bool SR = false>
-__global__ void __launch_bounds__(128) k_step_rows(const __grid_constant__ StepArgs<S> a) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int z = blockIdx.y, y = blockIdx.z;
+  chain_wait();
   bump_step_counter<SR>(a);
-  if (x >= a.g.nx) return;
-  step_node_at<S, COLL, LES, SR>(a, RowAddr<S>(a, x, y, z), x, y, z);
+  const FlatItem i = flat_item(a);
+  const bool faces = __any_sync(0xffffffffu, i.face_row);
+  if (!i.in) return;
+  paired_word<S, COLL, LES, SR>(a, i.x, i.y, i.z, faces);
 }
 
 // class of every node from the caller's mask (nonzero = solid); out may not

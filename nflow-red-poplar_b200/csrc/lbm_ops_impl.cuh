@@ -109,7 +109,7 @@ int ops_aa_macro(lbm_domain* d) {
   const int layout =
       d->cur ? kAASwapped : (d->post_direct ? kAANaturalComplete : kAANaturalPending);
   const dim3 b = block_of(d->g.nx), gr = grid_of(d->g, b);
-  k_aa_macro<S><<<gr, b, 0, d->stream>>>(m, layout);
+  launch_chained(k_aa_macro<S>, gr, b, d->stream, m, layout);
   CK(cudaGetLastError());
   return LBM_OK;
 }
@@ -119,30 +119,23 @@ int ops_run_aa(lbm_domain* d, int nsteps) {
   return with_model<S>(d, [&](auto coll, auto les) -> int {
     constexpr int C = decltype(coll)::value;
     constexpr bool L = decltype(les)::value;
-    const dim3 b = block_of(d->g.nx), gr = grid_of(d->g, b);
     auto args = [&](long long k, bool den, int neighbor) {
       return aa_args<S>(d, k, den, neighbor);
     };
-    // paired / quad rows (16-bit): k_aa_words, one word of two / four nodes
-    // per thread, except the first step after the initial state (a local
-    // step, whose slots are all at the node: the per-node step over the
-    // domain's rows)
     // quad rows (16-bit): k_aa_words, one word of four nodes per thread,
     // except the first step after the initial state (a local step, whose
     // slots are all at the node: the per-node step over quad rows)
     [[maybe_unused]] bool words = false;
-    [[maybe_unused]] dim3 bw(1, 1, 1), gw(1, 1, 1), gn(1, 1, 1);
+    const dim3 bf(kFlat);
+    const dim3 ga((unsigned)(((long long)d->g.px * d->g.nz + kFlat - 1) / kFlat), d->g.ny, 1);
+    [[maybe_unused]] dim3 gw(1, 1, 1), gn(1, 1, 1);
     if constexpr (kDev<S>) {
       if (d->g.rows != kRowsPlain) {
         if (!aa_words_apply(d->g))
           return set_error(LBM_ERR_INVALID, "AA domain rows without the word step");
         words = true;
-        const int nw = d->g.px / 4;
-        bw = block_of(nw);
-        gw = dim3((nw + bw.x - 1) / bw.x, d->g.nz, d->g.ny);  // local step: every row
-        // neighbour step: rows off the faces, then the face rows
-        const int fz = (aa_face_rows(d->g) + d->g.nz - 3) / (d->g.nz - 2);
-        gn = dim3(gw.x, d->g.nz - 2, d->g.ny - 2 + fz);
+        gw = flat_grid(d->g);
+        gn = aa_neighbor_grid(d->g);
         // channels: the buffer of the x-face values (k_aa_xface_rules)
         if (d->g.casetype == CHANNEL && !d->xrule)
           CK(cudaMalloc(&d->xrule, (size_t)10 * d->g.ny * d->g.nz * sizeof(float)));
@@ -158,32 +151,35 @@ int ops_run_aa(lbm_domain* d, int nsteps) {
             aw.xrule = d->xrule;
             if (aw.sr) {
               if (nb)
-                k_aa_words<S, C, L, true, 1, 2><<<gn, bw, 0, st>>>(aw, entry);
+                launch_chained(k_aa_words<S, C, L, true, 1>, gn, bf, st, aw, entry);
               else
-                k_aa_words<S, C, L, true, 0, 2><<<gw, bw, 0, st>>>(aw, entry);
+                launch_chained(k_aa_words<S, C, L, true, 0>, gw, bf, st, aw, entry);
             } else {
               if (nb)
-                k_aa_words<S, C, L, false, 1, 2><<<gn, bw, 0, st>>>(aw, entry);
+                launch_chained(k_aa_words<S, C, L, false, 1>, gn, bf, st, aw, entry);
               else
-                k_aa_words<S, C, L, false, 0, 2><<<gw, bw, 0, st>>>(aw, entry);
+                launch_chained(k_aa_words<S, C, L, false, 0>, gw, bf, st, aw, entry);
             }
           } else {
-            k_aa_step<S, C, L, 0><<<gr, b, 0, st>>>(a, entry);
+            StepArgs<S> an = a;  // one node per item
+            an.ri = d->g.px;
+            an.mrow = ~0ull / (unsigned long long)an.ri + 1;
+            launch_chained(k_aa_step<S, C, L, 0>, ga, bf, st, an, entry);
           }
           if (d->xrule) {
             // the next step's x-face values, from the face planes this step wrote
             StepArgs<S> fa = a;
             fa.prho_in = a.prho_out;
             fa.pu_in = a.pu_out;
-            k_aa_xface_rules<S><<<gx, 128, 0, st>>>(fa, d->xrule);
+            launch_chained(k_aa_xface_rules<S>, dim3(gx), dim3(128), st, fa, d->xrule);
           }
           return;
         }
       }
       if (nb)
-        k_aa_step<S, C, L, 1><<<gr, b, 0, st>>>(a, entry);
+        launch_chained(k_aa_step<S, C, L, 1>, ga, bf, st, a, entry);
       else
-        k_aa_step<S, C, L, 0><<<gr, b, 0, st>>>(a, entry);
+        launch_chained(k_aa_step<S, C, L, 0>, ga, bf, st, a, entry);
     };
     auto one = [&](bool den) {
       const long long k = d->step + 1;

@@ -38,13 +38,10 @@
 //   - rows on a y or z face: a population whose donor row is outside reads
 //     the node's own word of plane q and takes each node's wall rule; one
 //     whose destination row is outside writes the node's own word of plane
-//     opp q with each node's wall value (aa_wall).  The test is uniform along
-//     the row.
+//     opp q with each node's wall value (aa_wall).
 // No word is read outside its plane's rows: a seam word is addressed in its
 // own row, never one word past the row.
 #pragma once
-#include <type_traits>
-
 #include "lbm_kernels.cuh"
 
 namespace lbm {
@@ -66,14 +63,10 @@ __device__ __forceinline__ void st_w2(void* p, uint32_t v) {
   *reinterpret_cast<unsigned short*>(p) = (unsigned short)v;
 }
 
-// Resident threads per SM the register budgets are sized for: the quad step
-// (two F2 halves per thread, 128 registers) and the paired AA step (one F2
-// half, 64 registers).
+// Resident threads per SM the register budget is sized for (two F2 halves per
+// thread, 128 registers).
 #ifndef LBM_QUAD_THREADS_PER_SM
 #define LBM_QUAD_THREADS_PER_SM 512
-#endif
-#ifndef LBM_AA_PAIRED_THREADS_PER_SM
-#define LBM_AA_PAIRED_THREADS_PER_SM 1024
 #endif
 
 // index of population q (c_x = +-1) among the five with its c_x
@@ -97,6 +90,7 @@ __host__ __device__ constexpr int xface_index(int q) {
 template <class S>
 __global__ void __launch_bounds__(128) k_aa_xface_rules(const __grid_constant__ StepArgs<S> a,
                                                         float* __restrict__ out) {
+  chain_wait();
   const int ni = (a.g.ny - 2) * (a.g.nz - 2);
   const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (i >= 2 * ni) return;
@@ -117,213 +111,166 @@ __global__ void __launch_bounds__(128) k_aa_xface_rules(const __grid_constant__ 
   });
 }
 
-// The wall rule of boundary_value (fixed wall: the value itself; moving
-// wall: minus the lid term) for population q at a wall node of type t.
-template <class S, int q>
-__device__ __forceinline__ RealOf<S> wall_value(const StepArgs<S>& a, int t, RealOf<S> fo) {
-  using R = RealOf<S>;
-  if (t != NODE_MOVINGWALL) return fo;
-  constexpr int d = opp(q);
-  R eu = add_rn(add_rn(mul_rn(R(cx(d)), a.ulx), mul_rn(R(cy(d)), a.uly)), mul_rn(R(cz(d)), a.ulz));
-  R term = mul_rn(mul_rn(mul_rn(R(6), weight<R>(d)), a.rho0), eu);
-  return sub_rn(fo, term);
-}
-
-// a word of NH 32-bit halves (NH = 1: paired rows, 2: quad rows)
-template <int NH>
-using WordOf = typename std::conditional<NH == 1, uint32_t, uint2>::type;
-template <int h>
-__device__ __forceinline__ uint32_t& half_of(uint32_t& w) {
-  return w;
-}
-template <int h>
-__device__ __forceinline__ uint32_t& half_of(uint2& w) {
-  return h ? w.y : w.x;
-}
-__device__ __forceinline__ uint32_t ld_word(const void* p, uint32_t*) {
-  return *reinterpret_cast<const uint32_t*>(p);
-}
-__device__ __forceinline__ uint2 ld_word(const void* p, uint2*) { return ld_w8(p); }
-__device__ __forceinline__ void st_word(void* p, uint32_t v) { st_w4(p, v); }
-__device__ __forceinline__ void st_word(void* p, uint2 v) { st_w8(p, v); }
-
-// One AA step (NB = 0 local, 1 neighbour) of the 2 NH nodes of word w of
-// row (y, z), in paired rows (NH = 1: word w holds the nodes w, w + H) or
-// quad rows (NH = 2: see above).  Slot tables as for the per-node AA step
-// (aa_args with a.off[q] = 2 NH c_x + px (c_z + nz c_y)): local srcd[q] =
-// plane q, dstq[q] = plane opp q; neighbour srcd[q] = plane opp q - off_q,
-// dstq[q] = plane q + off_q; srcq[q] = plane q.  entry (local steps):
-// kAAPending or kAAComplete (the first step after the initial state is the
-// per-node step's).  In paired rows the seams are those of the pull step:
-// node H - 1 (lo of word H - 1) and node H (hi of word 0) are x neighbours,
-// node 0 is the lo of word 0 and node nx - 1 the hi of word H - 1.
-// FACE (neighbour step): the row lies on a y or z face, so that some
+// One AA step (NB = 0 local, 1 neighbour) of the four nodes of word w of row
+// (y, z).  Slot tables as for the per-node AA step (aa_args with a.off[q] =
+// 4 c_x + px (c_z + nz c_y)): local srcd[q] = plane q, dstq[q] = plane opp q;
+// neighbour srcd[q] = plane opp q - off_q, dstq[q] = plane q + off_q; srcq[q] =
+// plane q.  entry (local steps): kAAPending or kAAComplete (the first step
+// after the initial state is the per-node step's).
+// FACE (neighbour step): the row may lie on a y or z face, so that some
 // populations' donor or destination rows are outside the box; the rows off
-// the faces are stepped by a launch without that code (FACE = false), the
-// face rows by their own launch (k_aa_face_rows), which keeps each kernel's
-// code short.
-template <class S, int COLL, bool LES, bool SR, int NB, int NH, bool FACE>
+// the faces are stepped by CTAs without that code (FACE = false).
+template <class S, int COLL, bool LES, bool SR, int NB, bool FACE>
 __device__ __forceinline__ void aa_word(const StepArgs<S>& a, int w, int y, int z, int entry) {
-  static_assert(kDev<S>, "paired and quad rows are 16-bit layouts");
+  static_assert(kDev<S>, "quad rows are a 16-bit layout");
   static_assert(NB || !FACE, "face rows matter to the neighbour step only");
-  using W = WordOf<NH>;
-  const int H = a.g.px >> 1, D = a.g.px >> 2;
-  const int NW = a.g.px / (2 * NH);                    // words per row
-  const int e = 2 * NH * w + a.g.px * (z + a.g.nz * y);  // slot 0 of the word
-  const bool seam_lo = w == 0, seam_hi = w == NW - 1;
+  const int D = a.g.px >> 2, H = a.g.px >> 1;
+  const int e = 4 * w + a.g.px * (z + a.g.nz * y);  // slot 0 of the word
+  const bool seam_lo = w == 0, seam_hi = w == D - 1;
   // donor / destination row of population q inside the box (rows off a
   // face: always)
   auto row_in = [&](int dy, int dz) {
     if constexpr (!FACE) return true;
     return (unsigned)(y + dy) < (unsigned)a.g.ny && (unsigned)(z + dz) < (unsigned)a.g.nz;
   };
-  W v[Q];
+  uint2 v[Q];
   if constexpr (!NB) {
     static_for<0, Q>([&](auto qc) {
       constexpr int q = decltype(qc)::value;
-      v[q] = ld_word(a.srcd[q] + e, (W*)nullptr);
+      v[q] = ld_w8(a.srcd[q] + e);
     });
   } else {
     static_for<0, Q>([&](auto qc) {
       constexpr int q = decltype(qc)::value;
-      if (row_in(-cy(q), -cz(q))) {
-        // the donor word w - c_x, or across the seam the word at the other
-        // end of the same donor row (px elements away)
-        int adj = 0;
-        if constexpr (cx(q) == 1) adj = seam_lo ? a.g.px : 0;
-        if constexpr (cx(q) == -1) adj = seam_hi ? -a.g.px : 0;
-        v[q] = ld_word(a.srcd[q] + (e + adj), (W*)nullptr);
-      } else {
-        v[q] = ld_word(a.srcq[q] + e, (W*)nullptr);  // own slots (x, q): f*_{opp q}
-      }
+      // the donor word w - c_x, or across the seam the word at the other end
+      // of the same donor row (px elements away); a donor row outside: the
+      // own slots (x, q), which hold f*_{opp q}
+      int adj = 0;
+      if constexpr (cx(q) == 1) adj = seam_lo ? a.g.px : 0;
+      if constexpr (cx(q) == -1) adj = seam_hi ? -a.g.px : 0;
+      v[q] = ld_w8(row_in(-cy(q), -cz(q)) ? a.srcd[q] + (e + adj) : a.srcq[q] + e);
     });
-    if (seam_lo || seam_hi) {
+    // seam words: the own word of the five populations is fetched for all of
+    // them before the first is used (one memory latency; fetched one after
+    // the other they made a 32^3 neighbour step 3.5 times its local step)
+    if (seam_lo) {
+      uint2 own[Q];
       static_for<0, Q>([&](auto qc) {
         constexpr int q = decltype(qc)::value;
-        if constexpr (cx(q) != 0) {
-          if (((cx(q) == 1 && seam_lo) || (cx(q) == -1 && seam_hi)) &&
-              row_in(-cy(q), -cz(q))) {
-            const W X = v[q];
-            const W own = ld_word(a.srcq[q] + e, (W*)nullptr);
-            if constexpr (NH == 1) {
-              if constexpr (cx(q) == 1)
-                v[q] = __byte_perm(own, X, 0x5410);  // (own lo, node H - 1)
-              else
-                v[q] = __byte_perm(X, own, 0x7632);  // (node H, own hi)
-            } else {
-              if constexpr (cx(q) == 1) {
-                // quarters (own k0, X k0, X k1, X k2) in slot order k0 k2 | k1 k3
-                v[q].x = __byte_perm(own.x, X.y, 0x5410);
-                v[q].y = X.x;
-              } else {
-                // quarters (X k1, X k2, X k3, own k3)
-                v[q].x = X.y;
-                v[q].y = __byte_perm(X.x, own.y, 0x7632);
-              }
-            }
-          }
+        if constexpr (cx(q) == 1) own[q] = ld_w8(a.srcq[q] + e);
+      });
+      static_for<0, Q>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        if constexpr (cx(q) == 1) {
+          // quarters (own k0, X k0, X k1, X k2) in slot order k0 k2 | k1 k3
+          const uint2 X = v[q];
+          v[q].x = __byte_perm(own[q].x, X.y, 0x5410);
+          v[q].y = X.x;
+          if (!row_in(-cy(q), -cz(q))) v[q] = own[q];
+        }
+      });
+    }
+    if (seam_hi) {
+      uint2 own[Q];
+      static_for<0, Q>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        if constexpr (cx(q) == -1) own[q] = ld_w8(a.srcq[q] + e);
+      });
+      static_for<0, Q>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        if constexpr (cx(q) == -1) {
+          // quarters (X k1, X k2, X k3, own k3)
+          const uint2 X = v[q];
+          v[q].x = X.y;
+          v[q].y = __byte_perm(X.x, own[q].y, 0x7632);
+          if (!row_in(-cy(q), -cz(q))) v[q] = own[q];
         }
       });
     }
   }
-  if constexpr (SR) bump_step_counter<SR>(a);
   const uint32_t kstep = SR ? a.kctr[a.kpar] : 0u;
   // store of population q's word of results (slot order)
-  auto store = [&](auto qc, W r) {
+  auto store = [&](auto qc, uint2 r) {
     constexpr int q = decltype(qc)::value;
     if constexpr (!NB) {
-      st_word(a.dstq[q] + e, r);
+      st_w8(a.dstq[q] + e, r);
     } else {
       if (!row_in(cy(q), cz(q))) {
-        st_word(a.dst + (opp(q) * a.qs + e), r);  // own slots (x, opp q)
+        st_w8(a.dst + (opp(q) * a.qs + e), r);  // own slots (x, opp q)
       } else if (cx(q) == -1 && seam_lo) {
-        // the word across the seam is the last one of the destination row
+        // the word across the seam is the last one of the destination row:
+        // its slots k0 k2 k1 <- results k1 k3 k2; quarter 0 (x = 0) to its
+        // own slot
         S* wd = a.dstq[q] + (e + a.g.px);
-        if constexpr (NH == 1) {
-          st_w2(wd, r >> 16);                               // node H -> H - 1
-          st_w2(a.dst + (opp(q) * a.qs + e), r & 0xffffu);  // node 0: own slot
-        } else {
-          // its slots k0 k2 k1 <- results k1 k3 k2; quarter 0 (x = 0) to
-          // its own slot
-          st_w4(wd, r.y);
-          st_w2(wd + 2, r.x >> 16);
-          st_w2(a.dst + (opp(q) * a.qs + e), r.x & 0xffffu);
-        }
+        st_w4(wd, r.y);
+        st_w2(wd + 2, r.x >> 16);
+        st_w2(a.dst + (opp(q) * a.qs + e), r.x & 0xffffu);
       } else if (cx(q) == 1 && seam_hi) {
-        // the word across the seam is the first one of the destination row
+        // the word across the seam is the first one of the destination row:
+        // its slots k2 k1 k3 <- results k0 k1 k2; quarter 3 (x = nx - 1) to
+        // its own slot
         S* wd = a.dstq[q] + (e - a.g.px);
-        if constexpr (NH == 1) {
-          st_w2(wd + 1, r & 0xffffu);                           // node H - 1 -> H
-          st_w2(a.dst + (opp(q) * a.qs + e + 1), r >> 16);      // node nx - 1: own slot
-        } else {
-          // its slots k2 k1 k3 <- results k0 k1 k2; quarter 3 (x = nx - 1)
-          // to its own slot
-          st_w4(wd + 2, r.x);
-          st_w2(wd + 1, r.y & 0xffffu);
-          st_w2(a.dst + (opp(q) * a.qs + e + 3), r.y >> 16);
-        }
+        st_w4(wd + 2, r.x);
+        st_w2(wd + 1, r.y & 0xffffu);
+        st_w2(a.dst + (opp(q) * a.qs + e + 3), r.y >> 16);
       } else {
-        st_word(a.dstq[q] + e, r);
+        st_w8(a.dstq[q] + e, r);
       }
     }
   };
   // channels: the x-face lanes of this word take the values of
   // k_aa_xface_rules (node 0: lo lane of half 0 of word 0, c_x = +1
-  // populations; node nx - 1: hi lane of the last half of the last word,
-  // c_x = -1 populations)
+  // populations; node nx - 1: hi lane of half 1 of the last word, c_x = -1
+  // populations)
   auto xface_lanes = [&](F2 (&f)[Q], int hb) {
     const int P = a.g.ny * a.g.nz, yz = y * a.g.nz + z;
-    static_for<0, Q>([&](auto qc) {
-      constexpr int q = decltype(qc)::value;
-      if constexpr (cx(q) == 1) {
-        if (hb == 0 && seam_lo) f[q].v.x = a.xrule[xface_index(q) * P + yz];
-      } else if constexpr (cx(q) == -1) {
-        if (hb == NH - 1 && seam_hi) f[q].v.y = a.xrule[(5 + xface_index(q)) * P + yz];
-      }
-    });
+    if (hb == 0 && seam_lo) {
+      static_for<0, Q>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        if constexpr (cx(q) == 1) f[q].v.x = a.xrule[xface_index(q) * P + yz];
+      });
+    }
+    if (hb == 1 && seam_hi) {
+      static_for<0, Q>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        if constexpr (cx(q) == -1) f[q].v.y = a.xrule[(5 + xface_index(q)) * P + yz];
+      });
+    }
   };
+  // the cavity's lid, the only nodes of a face row whose rule changes the
+  // value: y = ny - 1 off its edges
+  [[maybe_unused]] const bool lid_row =
+      FACE && a.g.casetype == CAVITY && y == a.g.ny - 1 && z > 0 && z < a.g.nz - 1;
   // the halves, each a compile-time pass: half hb holds the nodes
-  // (w + hb D, w + hb D + H); every pass but the last leaves its packed
-  // results in its half of v[q], the last stores each population's word as
-  // soon as its result is known
+  // (w + hb D, w + hb D + H); the first leaves its packed results in its half
+  // of v[q], the second stores each population's word as soon as its result
+  // is known
   auto pass = [&](auto hbc) {
     constexpr int hb = decltype(hbc)::value;
     const int xlo = w + hb * D, xhi = xlo + H;
+    [[maybe_unused]] const bool lid_lo = lid_row && !(hb == 0 && seam_lo);
+    [[maybe_unused]] const bool lid_hi = lid_row && !(hb == 1 && seam_hi);
     F2 f[Q];
     static_for<0, Q>([&](auto qc) {
       constexpr int q = decltype(qc)::value;
-      f[q] = unpack_pair<S>(half_of<hb>(v[q]), a.inv_scale);
+      f[q] = unpack_pair<S>(hb ? v[q].y : v[q].x, a.inv_scale);
     });
-    [[maybe_unused]] int tlo = NODE_FLUID, thi = NODE_FLUID;
-    if constexpr (NB) {
-      // boundary rules of the donors outside the box.  Face rows: each
-      // node's wall rule (rows on a y or z face hold walls only: the lid,
-      // and fixed walls, which a channel's side faces keep over its inlet
-      // and outlet; their x faces are fixed walls, whose rule is the value
-      // itself).  Rows off the faces: the x faces (node 0, the lo lane of
-      // the first half of word 0; node nx - 1, the hi lane of the last half
-      // of the last word), whose rule is the value itself for the cavity's
-      // fixed walls and, for the channel's inlet and outlet, the value
-      // k_aa_xface_rules left for this step.
-      if constexpr (FACE) {
-        tlo = node_type(a.g, xlo, y, z);
-        thi = node_type(a.g, xhi, y, z);
+    if constexpr (FACE) {
+      if (lid_row) {
         static_for<0, Q>([&](auto qc) {
           constexpr int q = decltype(qc)::value;
-          if (!row_in(-cy(q), -cz(q))) {
-            f[q].v.x = wall_value<S, q>(a, tlo, f[q].v.x);
-            f[q].v.y = wall_value<S, q>(a, thi, f[q].v.y);
+          if constexpr (cy(q) == -1) {
+            if (lid_lo) f[q].v.x = aa_wall<S>(a, NODE_MOVINGWALL, f[q].v.x, opp(q));
+            if (lid_hi) f[q].v.y = aa_wall<S>(a, NODE_MOVINGWALL, f[q].v.y, opp(q));
           }
         });
-      } else if (a.xrule && (seam_lo || seam_hi)) {
-        xface_lanes(f, hb);
       }
     } else {
-      // pending natural slots of the channel's inlet and outlet nodes: the
-      // values k_aa_xface_rules left for this step
-      if (entry == kAAPending && a.xrule && y > 0 && y < a.g.ny - 1 && z > 0 &&
-          z < a.g.nz - 1 && (seam_lo || seam_hi))
-        xface_lanes(f, hb);
+      // channels: rows off the faces (neighbour step), the pending natural
+      // slots of the inlet and outlet nodes (local step)
+      const bool off_face = NB || (entry == kAAPending && y > 0 && y < a.g.ny - 1 && z > 0 &&
+                                   z < a.g.nz - 1);
+      if (a.xrule && off_face && (seam_lo || seam_hi)) xface_lanes(f, hb);
     }
     PairState<F2> ps;
     make_pairs<F2, true>(f, ps);
@@ -337,29 +284,24 @@ __device__ __forceinline__ void aa_word(const StepArgs<S>& a, int w, int y, int 
     if constexpr (SR) h = sr_hash((uint32_t)(xlo + H * (z + a.g.nz * y)), kstep, a.sr_seed);
     collide_node<S, COLL, LES, true, F2>(f, ps, ux, uy, uz, inv_rho, a, [&](auto qc, F2 r) {
       constexpr int q = decltype(qc)::value;
-      if constexpr (FACE) {
-        if (!row_in(cy(q), cz(q))) {
-          // destination row outside: the wall value into the node's own slot
-          r.v.x = aa_wall<S>(a, tlo, r.v.x, q);
-          r.v.y = aa_wall<S>(a, thi, r.v.y, q);
-        }
+      if constexpr (FACE && cy(q) == 1) {
+        // destination row outside: the wall value into the node's own slot
+        if (lid_lo) r.v.x = aa_wall<S>(a, NODE_MOVINGWALL, r.v.x, q);
+        if (lid_hi) r.v.y = aa_wall<S>(a, NODE_MOVINGWALL, r.v.y, q);
       }
       uint32_t p;
       if constexpr (SR)
         p = pack_pair_sr<S>(r, a.scale, sr_bits<q>(h));
       else
         p = pack_pair<S>(r, a.scale);
-      if constexpr (hb < NH - 1) {
-        half_of<hb>(v[q]) = p;
-      } else {
-        W out = v[q];
-        half_of<hb>(out) = p;
-        store(qc, out);
-      }
+      if constexpr (hb == 0)
+        v[q].x = p;
+      else
+        store(qc, make_uint2(v[q].x, p));
     });
   };
   pass(std::integral_constant<int, 0>{});
-  if constexpr (NH == 2) pass(std::integral_constant<int, 1>{});
+  pass(std::integral_constant<int, 1>{});
 }
 
 // number of rows on a y or z face: 2 nz at y = 0 and y = ny - 1, then
@@ -368,43 +310,50 @@ __host__ __device__ __forceinline__ int aa_face_rows(const Geometry& g) {
   return 2 * g.nz + 2 * (g.ny - 2);
 }
 
-// Local step: grid = (ceil(NW / b), nz, ny), every row.  Neighbour step:
-// grid = (ceil(NW / b), nz - 2, ny - 2 + FZ), FZ = ceil(aa_face_rows /
-// (nz - 2)): the rows off the y and z faces, then the face rows in the
-// trailing CTAs (a CTA-uniform branch into the code with the face rules,
-// so the hot code of the interior rows stays short and the face rows fill
-// the grid's tail).  NW = px / (2 NH) words per row, b = NW rounded up to a
-// multiple of 32 and at most 128 threads, one word per thread.  In the
-// neighbour step the two seam words of a row (0 and NW - 1) are taken by
-// the row's first two threads, so only the row's first warp diverges into
-// the seam code.
-template <class S, int COLL, bool LES, bool SR, int NB, int NH>
-__global__ void __launch_bounds__(128, (NH == 2 ? LBM_QUAD_THREADS_PER_SM
-                                                : LBM_AA_PAIRED_THREADS_PER_SM) / 128)
+// Neighbour step: CTA rows of the rows off the faces (blockIdx.y < ny - 2:
+// plane 1 + blockIdx.y, its nz - 2 inner rows one behind the other), then the
+// face rows, also one behind the other, in trailing CTAs (a CTA-uniform
+// branch into the code with the face rules, so the hot code of the inner rows
+// stays short and the face rows fill the grid's tail).
+inline dim3 aa_neighbor_grid(const Geometry& g) {
+  const long long D = g.px / 4, inner = D * (g.nz - 2), face = D * aa_face_rows(g);
+  const long long fc = (face + 127) / 128, room = 65535 - (g.ny - 2);  // CTA rows left
+  long long gx = (inner + 127) / 128;
+  if (gx * room < fc) gx = (fc + room - 1) / room;
+  return dim3((unsigned)gx, (unsigned)(g.ny - 2 + (fc + gx - 1) / gx), 1);
+}
+
+// Local step: grid = flat_grid, every row.  Neighbour step: grid =
+// aa_neighbor_grid.  One word per thread, CTAs of 128 threads over words of
+// consecutive rows (flat_item).
+template <class S, int COLL, bool LES, bool SR, int NB>
+__global__ void __launch_bounds__(128, LBM_QUAD_THREADS_PER_SM / 128)
     k_aa_words(const __grid_constant__ StepArgs<S> a, int entry) {
-  const int NW = a.g.px / (2 * NH);
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= NW) return;
+  chain_wait();
+  bump_step_counter<SR>(a);
   if constexpr (!NB) {
-    aa_word<S, COLL, LES, SR, 0, NH, false>(a, t, blockIdx.z, blockIdx.y, entry);  // y, z
+    const FlatItem i = flat_item(a);
+    if (i.in) aa_word<S, COLL, LES, SR, 0, false>(a, i.x, i.y, i.z, entry);
+  } else if ((int)blockIdx.y < a.g.ny - 2) {
+    const unsigned t = blockIdx.x * 128u + threadIdx.x;
+    const int r = (int)fastdiv(t, a.mrow);
+    if (r < a.g.nz - 2)
+      aa_word<S, COLL, LES, SR, 1, false>(a, (int)t - r * a.ri, (int)blockIdx.y + 1, r + 1, entry);
   } else {
-    const int w = t == 0 ? 0 : (t == 1 ? NW - 1 : t - 1);
-    if ((int)blockIdx.z < a.g.ny - 2) {
-      aa_word<S, COLL, LES, SR, 1, NH, false>(a, w, blockIdx.z + 1, blockIdx.y + 1, entry);
+    const unsigned c = (blockIdx.y - (unsigned)(a.g.ny - 2)) * gridDim.x + blockIdx.x;
+    const unsigned t = c * 128u + threadIdx.x;
+    const int r = (int)fastdiv(t, a.mrow);
+    if (r >= aa_face_rows(a.g)) return;
+    int y, z;
+    if (r < 2 * a.g.nz) {
+      y = r < a.g.nz ? 0 : a.g.ny - 1;
+      z = r < a.g.nz ? r : r - a.g.nz;
     } else {
-      const int r = ((int)blockIdx.z - (a.g.ny - 2)) * (a.g.nz - 2) + (int)blockIdx.y;
-      if (r >= aa_face_rows(a.g)) return;
-      int y, z;
-      if (r < 2 * a.g.nz) {
-        y = r < a.g.nz ? 0 : a.g.ny - 1;
-        z = r % a.g.nz;
-      } else {
-        const int r2 = r - 2 * a.g.nz;
-        z = r2 < a.g.ny - 2 ? 0 : a.g.nz - 1;
-        y = 1 + r2 % (a.g.ny - 2);
-      }
-      aa_word<S, COLL, LES, SR, 1, NH, true>(a, w, y, z, entry);
+      const int r2 = r - 2 * a.g.nz;
+      z = r2 < a.g.ny - 2 ? 0 : a.g.nz - 1;
+      y = 1 + (r2 < a.g.ny - 2 ? r2 : r2 - (a.g.ny - 2));
     }
+    aa_word<S, COLL, LES, SR, 1, true>(a, (int)t - r * a.ri, y, z, entry);
   }
 }
 

@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(TmaCfg<S>::THREADS, 1)
       if (x < x0 || x >= x0 + C::TX || x >= nx || (c >= 2 && x < 2)) continue;
       const int pair = x & ~1;
       if (pair >= 1 && pair + 1 <= nx - 2) continue;  // a consumer's interior pair
-      step_node<S, COLL, LES>(a, x, y, z);
+      step_node<S, COLL, LES>(a, x, y, z, true);
     }
     return;
   }
@@ -248,8 +248,8 @@ __global__ void __launch_bounds__(TmaCfg<S>::THREADS, 1)
         });
       } else if (face_row) {
         // a row of boundary nodes: the per-node path with the boundary rules
-        step_node<S, COLL, LES>(a, x, y, z);
-        if (two) step_node<S, COLL, LES>(a, x + 1, y, z);
+        step_node<S, COLL, LES>(a, x, y, z, true);
+        if (two) step_node<S, COLL, LES>(a, x + 1, y, z, true);
       }
       // else: an x-face pair of an interior row, done by the boundary warp
     }
