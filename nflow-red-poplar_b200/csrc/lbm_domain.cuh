@@ -254,6 +254,7 @@ StepArgs<S> make_args(const lbm_domain* d, const void* src, void* dst, long long
   }
   a.g = d->g;
   a.ri = row_items(d->g);
+  a.rev = src && src == d->lat[1];
   a.mrow = ~0ull / (unsigned long long)a.ri + 1;
   a.tau = R(d->in.m_dTau);
   const double cs = (double)d->in.m_dSmagorinsky;
@@ -310,6 +311,7 @@ StepArgs<S> aa_args(const lbm_domain* d, long long k, bool den, int neighbor) {
   }
   if (den) a.den_out = d->den[(k - 1) & 1];
   a.aa_step = 1 + neighbor;
+  a.rev = neighbor;
   return a;
 }
 
