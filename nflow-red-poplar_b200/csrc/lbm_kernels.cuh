@@ -216,11 +216,6 @@ struct StepArgs {
   int kpar;
   int sr;
   unsigned sr_seed;
-  // channel on quad rows: the inlet / outlet values this step takes for the
-  // populations whose donor lies outside the box at x = 0 (c_x = +1) and
-  // x = nx - 1 (c_x = -1), [2][5][ny*nz], computed after the step before
-  // (k_aa_xface_rules)
-  const float* xrule;
 };
 
 // First statement of every kernel of the step chain (launch_chained): let the
@@ -937,7 +932,8 @@ struct AADst {
 // z face; without it only x = 0 and x = nx - 1 are looked at, which is what
 // most of the warps need that come here.  (With one form for both the 256^3
 // FP32 neighbour step took 516 us, with two 430 us.)
-template <class S, int COLL, bool LES, bool ROWS>
+// MACRO: rho and u only.
+template <class S, int COLL, bool LES, bool ROWS, bool MACRO>
 __device__ __forceinline__ void aa_neighbor_face_node(const StepArgs<S>& a, int x, int y, int z,
                                                       int cell) {
   using R = RealOf<S>;
@@ -965,6 +961,7 @@ __device__ __forceinline__ void aa_neighbor_face_node(const StepArgs<S>& a, int 
   R ux, uy, uz;
   const R inv_rho = velocity<R>(ps, ux, uy, uz);
   write_macro<S>(a, x, y, z, ps.rho_full, ux, uy, uz);
+  if constexpr (MACRO) return;
   collide_node<S, COLL, LES, kFromPairs<S>, R>(f, ps, ux, uy, uz, inv_rho, a, [&](auto qc, R v) {
     constexpr int q = decltype(qc)::value;
     const bool out = !row_in(cy(q), cz(q)) || (cx(q) == -1 && xlo) || (cx(q) == 1 && xhi);
@@ -986,7 +983,9 @@ enum { kFacesNone = 0, kFacesX = 1, kFacesRow = 2 };
 
 // faces: the form of the neighbour step: kFacesNone, kFacesX (nodes at x = 0 or
 // x = nx - 1 among the warp's) or kFacesRow (nodes on a y or z face).
-template <class S, int COLL, bool LES>
+// MACRO: only rho and u of arF in the layout that step would read, for a.den_out
+// and a.ux_out.
+template <class S, int COLL, bool LES, bool MACRO = false>
 __device__ __forceinline__ void aa_step_node(const StepArgs<S>& a, int x, int y, int z,
                                              int neighbor, int entry, int faces) {
   using R = RealOf<S>;
@@ -995,9 +994,9 @@ __device__ __forceinline__ void aa_step_node(const StepArgs<S>& a, int x, int y,
   const int cell = neighbor ? x + a.g.px * (z + a.g.nz * y) : cell_of(a.g, x, y, z);
   if (neighbor && faces != kFacesNone) {
     if (faces == kFacesX)
-      aa_neighbor_face_node<S, COLL, LES, false>(a, x, y, z, cell);
+      aa_neighbor_face_node<S, COLL, LES, false, MACRO>(a, x, y, z, cell);
     else
-      aa_neighbor_face_node<S, COLL, LES, true>(a, x, y, z, cell);
+      aa_neighbor_face_node<S, COLL, LES, true, MACRO>(a, x, y, z, cell);
     return;
   }
   R f[Q];
@@ -1009,7 +1008,15 @@ __device__ __forceinline__ void aa_step_node(const StepArgs<S>& a, int x, int y,
   if (neighbor || entry != kAAFromInit) {
     if (!neighbor && entry == kAAPending && ((x == 0) | (x == a.g.nx - 1)))
       aa_open_face_rules<S>(f, a, x, y, z);
-    finish_node<S, COLL, LES>(f, a, ad, x, y, z);
+    if constexpr (MACRO) {
+      PairState<R> ps;
+      make_pairs<R, kDev<S>>(f, ps);
+      R ux, uy, uz;
+      velocity<R>(ps, ux, uy, uz);
+      write_macro<S>(a, x, y, z, ps.rho_full, ux, uy, uz);
+    } else {
+      finish_node<S, COLL, LES>(f, a, ad, x, y, z);
+    }
     return;
   }
   // the first step after the initial state
@@ -1053,35 +1060,22 @@ __global__ void __launch_bounds__(128, NB ? 7 : 9)
 }
 
 // rho and u of arF in the current AA layout, written through a.den_out /
-// a.ux_out...: the same arithmetic as the step kernels' side outputs.
-// layout: kAASwapped (after a local step), kAANaturalPending (after a
-// neighbour step), kAANaturalComplete.
-enum { kAANaturalComplete = 0, kAASwapped = 1, kAANaturalPending = 2 };
-
-template <class S>
+// a.ux_out...: the loads and the arithmetic of the step that would come next
+// (NB, entry: its kind and entry mode).
+template <class S, int NB>
 __global__ void __launch_bounds__(128) k_aa_macro(const __grid_constant__ StepArgs<S> a,
-                                                  int layout) {
+                                                  int entry) {
   chain_wait();
-  using R = RealOf<S>;
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int z = blockIdx.y, y = blockIdx.z;
-  if (x >= a.g.nx) return;
-  const int cell = cell_of(a.g, x, y, z);
-  R f[Q];
-  if (layout == kAASwapped) {
-    aa_pull_swapped<S>(f, a, x, y, z, cell);
-  } else {
-    static_for<0, Q>([&](auto qc) {
-      constexpr int q = decltype(qc)::value;
-      f[q] = ld(a.srcq[q] + cell, q, a.inv_scale);
-    });
-    if (layout == kAANaturalPending) aa_open_face_rules<S>(f, a, x, y, z);
+  const FlatItem i = flat_item(a);
+  int faces = kFacesNone;
+  if constexpr (NB) {
+    if (__any_sync(0xffffffffu, i.face_row))
+      faces = kFacesRow;
+    else if (__any_sync(0xffffffffu, (i.x == 0) | (i.x == a.g.nx - 1)))
+      faces = kFacesX;
   }
-  PairState<R> ps;
-  make_pairs<R, kDev<S>>(f, ps);
-  R ux, uy, uz;
-  velocity<R>(ps, ux, uy, uz);
-  write_macro<S>(a, x, y, z, ps.rho_full, ux, uy, uz);
+  if (!i.in) return;
+  aa_step_node<S, COLL_SRT, false, true>(a, i.x, i.y, i.z, NB, entry, faces);
 }
 
 enum { kExportPull = 0, kExportDirect = 1, kExportAASwapped = 2, kExportAANaturalPending = 3 };

@@ -101,15 +101,29 @@ int ops_run_pull(lbm_domain* d, int nsteps) {
 // from either layout; the face buffers are those of AA step s (k = s + 1)
 template <class S>
 int ops_aa_macro(lbm_domain* d) {
-  StepArgs<S> m = make_args<S>(d, d->lat[0], d->lat[0], d->step + 1);
+  StepArgs<S> m = aa_args<S>(d, d->step + 1, false, d->cur);
   m.den_out = d->den[d->step & 1];
   m.ux_out = d->ux;
   m.uy_out = d->uy;
   m.uz_out = d->uz;
-  const int layout =
-      d->cur ? kAASwapped : (d->post_direct ? kAANaturalComplete : kAANaturalPending);
-  const dim3 b = block_of(d->g.nx), gr = grid_of(d->g, b);
-  launch_chained(k_aa_macro<S>, gr, b, d->stream, m, layout);
+  const int entry = d->post_direct ? kAAComplete : kAAPending;
+  const dim3 bf(kFlat);
+  if constexpr (kDev<S>) {
+    if (d->g.rows == kRowsQuad) {
+      if (d->cur)
+        launch_chained(k_aa_words<S, COLL_SRT, false, false, 1, true>, aa_neighbor_grid(d->g), bf,
+                       d->stream, m, entry);
+      else
+        launch_chained(k_aa_words<S, COLL_SRT, false, false, 0, true>, flat_grid(d->g), bf,
+                       d->stream, m, entry);
+      CK(cudaGetLastError());
+      return LBM_OK;
+    }
+  }
+  if (d->cur)
+    launch_chained(k_aa_macro<S, 1>, flat_grid(d->g), bf, d->stream, m, entry);
+  else
+    launch_chained(k_aa_macro<S, 0>, flat_grid(d->g), bf, d->stream, m, entry);
   CK(cudaGetLastError());
   return LBM_OK;
 }
@@ -136,42 +150,28 @@ int ops_run_aa(lbm_domain* d, int nsteps) {
         words = true;
         gw = flat_grid(d->g);
         gn = aa_neighbor_grid(d->g);
-        // channels: the buffer of the x-face values (k_aa_xface_rules)
-        if (d->g.casetype == CHANNEL && !d->xrule)
-          CK(cudaMalloc(&d->xrule, (size_t)10 * d->g.ny * d->g.nz * sizeof(float)));
       }
     }
-    [[maybe_unused]] const unsigned gx =
-        (unsigned)((2 * (d->g.ny - 2) * (d->g.nz - 2) + 127) / 128);
     auto launch = [&](cudaStream_t st, const StepArgs<S>& a, int nb, int entry) {
       if constexpr (kDev<S>) {
         if (words) {
           if (entry != kAAFromInit) {
-            StepArgs<S> aw = a;
-            aw.xrule = d->xrule;
-            if (aw.sr) {
+            if (a.sr) {
               if (nb)
-                launch_chained(k_aa_words<S, C, L, true, 1>, gn, bf, st, aw, entry);
+                launch_chained(k_aa_words<S, C, L, true, 1>, gn, bf, st, a, entry);
               else
-                launch_chained(k_aa_words<S, C, L, true, 0>, gw, bf, st, aw, entry);
+                launch_chained(k_aa_words<S, C, L, true, 0>, gw, bf, st, a, entry);
             } else {
               if (nb)
-                launch_chained(k_aa_words<S, C, L, false, 1>, gn, bf, st, aw, entry);
+                launch_chained(k_aa_words<S, C, L, false, 1>, gn, bf, st, a, entry);
               else
-                launch_chained(k_aa_words<S, C, L, false, 0>, gw, bf, st, aw, entry);
+                launch_chained(k_aa_words<S, C, L, false, 0>, gw, bf, st, a, entry);
             }
           } else {
             StepArgs<S> an = a;  // one node per item
             an.ri = d->g.px;
             an.mrow = ~0ull / (unsigned long long)an.ri + 1;
             launch_chained(k_aa_step<S, C, L, 0>, ga, bf, st, an, entry);
-          }
-          if (d->xrule) {
-            // the next step's x-face values, from the face planes this step wrote
-            StepArgs<S> fa = a;
-            fa.prho_in = a.prho_out;
-            fa.pu_in = a.pu_out;
-            launch_chained(k_aa_xface_rules<S>, dim3(gx), dim3(128), st, fa, d->xrule);
           }
           return;
         }

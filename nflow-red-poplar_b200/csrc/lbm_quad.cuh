@@ -69,48 +69,6 @@ __device__ __forceinline__ void st_w2(void* p, uint32_t v) {
 #define LBM_QUAD_THREADS_PER_SM 512
 #endif
 
-// index of population q (c_x = +-1) among the five with its c_x
-__host__ __device__ constexpr int xface_index(int q) {
-  int j = 0;
-  for (int p = 1; p < q; ++p) j += cx(p) == cx(q);
-  return j;
-}
-
-// Channels on quad rows: after every AA step, the inlet / outlet values
-// that the next step takes for the populations whose donor lies outside the
-// box at the x faces of the interior rows: at x = 0 (inlet) the five with
-// c_x = +1, at x = nx - 1 (outlet) the five with c_x = -1.  In both AA
-// layouts the node's own slot (x, q) then holds f*_{opp q} (a pending
-// natural slot after a neighbour step, the own slot after a local step), and
-// the value is boundary_value of the node with the face planes the step
-// just wrote: a = the next step's arguments.  The step kernels read the
-// five values instead of evaluating the rule (FP64 arithmetic that only
-// two threads of a row would run): the same FP32 values, so the same bits.
-// grid = ceil(2 (ny - 2)(nz - 2) / 128) blocks of 128.
-template <class S>
-__global__ void __launch_bounds__(128) k_aa_xface_rules(const __grid_constant__ StepArgs<S> a,
-                                                        float* __restrict__ out) {
-  chain_wait();
-  const int ni = (a.g.ny - 2) * (a.g.nz - 2);
-  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (i >= 2 * ni) return;
-  const int face = i >= ni, r = face ? i - ni : i;
-  const int y = 1 + r / (a.g.nz - 2), z = 1 + r % (a.g.nz - 2);
-  const int x = face ? a.g.nx - 1 : 0;
-  const int P = a.g.ny * a.g.nz, yz = y * a.g.nz + z;
-  const int t = node_type(a.g, x, y, z);
-  const int cell = cell_of(a.g, x, y, z);
-  static_for<1, Q>([&](auto qc) {
-    constexpr int q = decltype(qc)::value;
-    if constexpr (cx(q) != 0) {
-      if ((cx(q) == 1) == (face == 0)) {
-        const RealOf<S> fo = ld(a.srcq[q] + cell, q, a.inv_scale);
-        out[(face * 5 + xface_index(q)) * P + yz] = (float)boundary_value<S, q>(a, t, fo, y, z);
-      }
-    }
-  });
-}
-
 // One AA step (NB = 0 local, 1 neighbour) of the four nodes of word w of row
 // (y, z).  Slot tables as for the per-node AA step (aa_args with a.off[q] =
 // 4 c_x + px (c_z + nz c_y)): local srcd[q] = plane q, dstq[q] = plane opp q;
@@ -120,7 +78,9 @@ __global__ void __launch_bounds__(128) k_aa_xface_rules(const __grid_constant__ 
 // FACE (neighbour step): the row may lie on a y or z face, so that some
 // populations' donor or destination rows are outside the box; the rows off
 // the faces are stepped by CTAs without that code (FACE = false).
-template <class S, int COLL, bool LES, bool SR, int NB, bool FACE>
+// MACRO: only rho and u of arF in the layout that step would read, for
+// a.den_out and a.ux_out.
+template <class S, int COLL, bool LES, bool SR, int NB, bool FACE, bool MACRO = false>
 __device__ __forceinline__ void aa_word(const StepArgs<S>& a, int w, int y, int z, int entry) {
   static_assert(kDev<S>, "quad rows are a 16-bit layout");
   static_assert(NB || !FACE, "face rows matter to the neighbour step only");
@@ -218,22 +178,24 @@ __device__ __forceinline__ void aa_word(const StepArgs<S>& a, int w, int y, int 
       }
     }
   };
-  // channels: the x-face lanes of this word take the values of
-  // k_aa_xface_rules (node 0: lo lane of half 0 of word 0, c_x = +1
-  // populations; node nx - 1: hi lane of half 1 of the last word, c_x = -1
-  // populations)
-  auto xface_lanes = [&](F2 (&f)[Q], int hb) {
-    const int P = a.g.ny * a.g.nz, yz = y * a.g.nz + z;
+  // channels: inlet and outlet rules of node 0 (lo lane of half 0 of word 0,
+  // c_x = +1 populations) and node nx - 1 (hi lane of half 1 of the last word,
+  // c_x = -1 populations), in rows off the faces: f holds the node's own
+  // f*_{opp q} there.  One lane of a row evaluates them; a kernel of its own
+  // after each step, which left the values for the next one, cost a launch
+  // and 10 scattered reads a row: 32^3 10.3 us a step against 4.8 here,
+  // 256x72x64 26.8 against 20.9, 512x128x128 148 against 142.5.
+  auto open_face_rules = [&](F2 (&f)[Q], int hb) {
     if (hb == 0 && seam_lo) {
       static_for<0, Q>([&](auto qc) {
         constexpr int q = decltype(qc)::value;
-        if constexpr (cx(q) == 1) f[q].v.x = a.xrule[xface_index(q) * P + yz];
+        if constexpr (cx(q) == 1) f[q].v.x = boundary_value<S, q>(a, NODE_INLET, f[q].v.x, y, z);
       });
     }
     if (hb == 1 && seam_hi) {
       static_for<0, Q>([&](auto qc) {
         constexpr int q = decltype(qc)::value;
-        if constexpr (cx(q) == -1) f[q].v.y = a.xrule[(5 + xface_index(q)) * P + yz];
+        if constexpr (cx(q) == -1) f[q].v.y = boundary_value<S, q>(a, NODE_OUTLET, f[q].v.y, y, z);
       });
     }
   };
@@ -270,16 +232,18 @@ __device__ __forceinline__ void aa_word(const StepArgs<S>& a, int w, int y, int 
       // slots of the inlet and outlet nodes (local step)
       const bool off_face = NB || (entry == kAAPending && y > 0 && y < a.g.ny - 1 && z > 0 &&
                                    z < a.g.nz - 1);
-      if (a.xrule && off_face && (seam_lo || seam_hi)) xface_lanes(f, hb);
+      if (a.g.casetype == CHANNEL && off_face) open_face_rules(f, hb);
     }
     PairState<F2> ps;
     make_pairs<F2, true>(f, ps);
     F2 ux, uy, uz;
     const F2 inv_rho = velocity<F2>(ps, ux, uy, uz);
-    if (a.den_out || a.ux_out || a.g.casetype == CHANNEL) {
+    // (channels: the nodes 1, nx - 1 and nx - 2 leave their state for the rules)
+    if (a.den_out || a.ux_out || (a.g.casetype == CHANNEL && (w == 1 || w >= D - 2))) {
       write_macro<S>(a, xlo, y, z, ps.rho_full.v.x, ux.v.x, uy.v.x, uz.v.x);
       write_macro<S>(a, xhi, y, z, ps.rho_full.v.y, ux.v.y, uy.v.y, uz.v.y);
     }
+    if constexpr (MACRO) return;
     [[maybe_unused]] uint32_t h = 0u;
     if constexpr (SR) h = sr_hash((uint32_t)(xlo + H * (z + a.g.nz * y)), kstep, a.sr_seed);
     collide_node<S, COLL, LES, true, F2>(f, ps, ux, uy, uz, inv_rho, a, [&](auto qc, F2 r) {
@@ -325,22 +289,22 @@ inline dim3 aa_neighbor_grid(const Geometry& g) {
 
 // Local step: grid = flat_grid, every row.  Neighbour step: grid =
 // aa_neighbor_grid.  One word per thread, CTAs of 128 threads over words of
-// consecutive rows (flat_item).
-template <class S, int COLL, bool LES, bool SR, int NB>
+// consecutive rows (flat_item).  MACRO: rho and u instead of the step.
+template <class S, int COLL, bool LES, bool SR, int NB, bool MACRO = false>
 __global__ void __launch_bounds__(128, LBM_QUAD_THREADS_PER_SM / 128)
     k_aa_words(const __grid_constant__ StepArgs<S> a, int entry) {
   chain_wait();
-  bump_step_counter<SR>(a);
+  if constexpr (!MACRO) bump_step_counter<SR>(a);
   if constexpr (!NB) {
     const FlatItem i = flat_item(a);
-    if (i.in) aa_word<S, COLL, LES, SR, 0, false>(a, i.x, i.y, i.z, entry);
+    if (i.in) aa_word<S, COLL, LES, SR, 0, false, MACRO>(a, i.x, i.y, i.z, entry);
   } else if ((int)blockIdx.y < a.g.ny - 2) {
     // backwards, as flat_item with a.rev: the local steps run forwards
     const unsigned t = (gridDim.x - 1 - blockIdx.x) * 128u + threadIdx.x;
     const int r = (int)fastdiv(t, a.mrow);
     if (r < a.g.nz - 2)
-      aa_word<S, COLL, LES, SR, 1, false>(a, (int)t - r * a.ri, a.g.ny - 2 - (int)blockIdx.y, r + 1,
-                                          entry);
+      aa_word<S, COLL, LES, SR, 1, false, MACRO>(a, (int)t - r * a.ri,
+                                                 a.g.ny - 2 - (int)blockIdx.y, r + 1, entry);
   } else {
     const unsigned c = (blockIdx.y - (unsigned)(a.g.ny - 2)) * gridDim.x + blockIdx.x;
     const unsigned t = c * 128u + threadIdx.x;
@@ -355,7 +319,7 @@ __global__ void __launch_bounds__(128, LBM_QUAD_THREADS_PER_SM / 128)
       z = r2 < a.g.ny - 2 ? 0 : a.g.nz - 1;
       y = 1 + (r2 < a.g.ny - 2 ? r2 : r2 - (a.g.ny - 2));
     }
-    aa_word<S, COLL, LES, SR, 1, true>(a, (int)t - r * a.ri, y, z, entry);
+    aa_word<S, COLL, LES, SR, 1, true, MACRO>(a, (int)t - r * a.ri, y, z, entry);
   }
 }
 
