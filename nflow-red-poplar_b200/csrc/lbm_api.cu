@@ -81,8 +81,9 @@ __global__ void __launch_bounds__(kDiagThreads)
     if (has_prev) v[4] += fabs(r - (double)den_prev[i]);
     const double u2 = a * a + b * b + c * c;
     v[5] += 0.5 * r * u2;
-    v[6] = fmax(v[6], sqrt(u2));
+    v[6] = fmax(v[6], u2);
   }
+  v[6] = sqrt(v[6]);  // the root is monotonic: of the largest only
   __shared__ double sh[8][kDiagThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int k = 0; k < 8; ++k) {
@@ -102,15 +103,24 @@ __global__ void __launch_bounds__(kDiagThreads)
   }
 }
 
-__global__ void k_diag_final(const double* __restrict__ partial, int nblocks,
-                             double* __restrict__ out) {
-  if (threadIdx.x < 8) {
-    const int k = threadIdx.x;
-    double x = 0.0;
-    for (int b = 0; b < nblocks; ++b)
-      x = (k == 6) ? fmax(x, partial[b * 8 + k]) : x + partial[b * 8 + k];
-    out[k] = x;
+// One block.  The sum runs over the blocks in order, so that it depends on
+// nothing but the data; what it waited for was one L2 latency per block, so all
+// threads bring a stretch of the partial sums into shared memory first.
+__global__ void __launch_bounds__(kDiagThreads)
+    k_diag_final(const double* __restrict__ partial, int nblocks, double* __restrict__ out) {
+  constexpr int kRun = 512;  // blocks of a stretch (32 KB)
+  __shared__ double sh[kRun * 8];
+  double x = 0.0;
+  const int k = threadIdx.x;
+  for (int b0 = 0; b0 < nblocks; b0 += kRun) {
+    const int n = min(kRun, nblocks - b0);
+    for (int i = threadIdx.x; i < n * 8; i += kDiagThreads) sh[i] = partial[b0 * 8 + i];
+    __syncthreads();
+    if (k < 8)
+      for (int b = 0; b < n; ++b) x = (k == 6) ? fmax(x, sh[b * 8 + k]) : x + sh[b * 8 + k];
+    __syncthreads();
   }
+  if (k < 8) out[k] = x;
 }
 
 }  // namespace lbm
@@ -374,7 +384,7 @@ int lbm_diagnostics(lbm_domain* d, double out[8]) {
   const long long k = d->step;
   k_diag_partial<<<d->diag_blocks, kDiagThreads, 0, d->stream>>>(
       d->den[k & 1], d->den[(k + 1) & 1], d->ux, d->uy, d->uz, d->N, k > 0 ? 1 : 0, d->partial);
-  k_diag_final<<<1, 32, 0, d->stream>>>(d->partial, d->diag_blocks, d->dout);
+  k_diag_final<<<1, kDiagThreads, 0, d->stream>>>(d->partial, d->diag_blocks, d->dout);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(out, d->dout, 8 * sizeof(double), cudaMemcpyDeviceToHost, d->stream));
   CK(cudaStreamSynchronize(d->stream));
