@@ -380,6 +380,9 @@ void launch_step(const lbm_domain* d, const StepArgs<S>& a, cudaStream_t st) {
       launch_chained(k_step<S, COLL, LES, true>, flat_grid(d->g), dim3(kFlat), st, a);
       return;
     }
+  } else if ((long long)Q * d->qs * (long long)sizeof(S) <= kOnceBytes) {
+    launch_chained(k_step<S, COLL, LES, false, true>, flat_grid(d->g), dim3(kFlat), st, a);
+    return;
   }
   launch_chained(k_step<S, COLL, LES, false>, flat_grid(d->g), dim3(kFlat), st, a);
 }

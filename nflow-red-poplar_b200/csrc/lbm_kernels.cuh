@@ -272,6 +272,22 @@ __device__ __forceinline__ RealOf<S> ld(const S* p, int, float inv_scale) {
   return StoreTraits<S>::load(p, inv_scale);
 }
 
+// The same from the source lattice of a pull step (ONCE: fetched as streaming
+// data).  The source is dead once read, so marking it lets the L2 keep what
+// the step writes for the next one, as long as one lattice about fits there:
+// us a step without -> with, FP32 80^3 11.1 -> 10.7, 96^3 21.3 -> 19.6, 128^3 (160 MB)
+// 50.2 -> 49.7; FP64 80^3 22.6 -> 20.6, 96^3 40.1 -> 38.5.  Beyond, a sector that two
+// warps share is gone before the second reads it: FP32 160^3 (311 MB) 99 -> 102,
+// 256^3 396 -> 417; the 16-bit kernels only lose (FP16 128^3 37.0 -> 39.9).
+constexpr long long kOnceBytes = 160ll << 20;  // largest lattice fetched that way
+template <class S, bool ONCE>
+__device__ __forceinline__ RealOf<S> ld_src(const S* p, int q, float inv_scale) {
+  if constexpr (ONCE)
+    return __ldcs(p);
+  else
+    return ld(p, q, inv_scale);
+}
+
 // Where the populations of a node live (cell = in-plane index of the node)
 // and the storage scales of the shifted 16-bit forms (g = h * inv_scale on
 // load, h = g * scale on store).  PlaneAddr takes the per-population plane pointers and
@@ -500,7 +516,7 @@ __device__ __forceinline__ void face_rules(RealOf<S> (&f)[Q], const StepArgs<S>&
 // warp that holds one, so that the warp does not run both.  (When each lane
 // took its own form, with the rules of every node type inlined 18 times, a
 // 16^3 FP32 step took 3.8 us, 64^3 9.3 us and 96^3 27.3 us; now 2.1, 6.7 and 22.4.)
-template <class S, class Addr>
+template <class S, bool ONCE = false, class Addr>
 __device__ __forceinline__ void pull(RealOf<S> (&f)[Q], const StepArgs<S>& a, const Addr& ad, int x,
                                      int y, int z, bool faces) {
   if (has_struct(a.g) && struct_class(a.g, x, y, z) != kSolidFree) {
@@ -508,7 +524,7 @@ __device__ __forceinline__ void pull(RealOf<S> (&f)[Q], const StepArgs<S>& a, co
   } else if (!faces) {
     static_for<0, Q>([&](auto qc) {
       constexpr int q = decltype(qc)::value;
-      f[q] = ld(ad.donor(q), q, ad.inv_scale());
+      f[q] = ld_src<S, ONCE>(ad.donor(q), q, ad.inv_scale());
     });
   } else {
     const bool xlo = x == 0, xhi = x == a.g.nx - 1;
@@ -517,7 +533,7 @@ __device__ __forceinline__ void pull(RealOf<S> (&f)[Q], const StepArgs<S>& a, co
       const bool row_out = (unsigned)(y - cy(q)) >= (unsigned)a.g.ny ||
                            (unsigned)(z - cz(q)) >= (unsigned)a.g.nz;
       const bool out = row_out || (cx(q) == 1 && xlo) || (cx(q) == -1 && xhi);
-      f[q] = ld(out ? ad.own(opp(q)) : ad.donor(q), q, ad.inv_scale());
+      f[q] = ld_src<S, ONCE>(out ? ad.own(opp(q)) : ad.donor(q), q, ad.inv_scale());
     });
     face_rules<S>(f, a, x, y, z,
                   (y == 0) | (y == a.g.ny - 1) | (z == 0) | (z == a.g.nz - 1));
@@ -668,7 +684,7 @@ __device__ __forceinline__ void finish_node(const RealOf<S> (&f)[Q], const StepA
 // LES, collision, store.  Shared by the single-domain and batched kernels,
 // so a domain gets the same bits alone and in a batch (only where the
 // arguments are held differs, not the arithmetic).
-template <class S, int COLL, bool LES, bool SR = false, class Addr>
+template <class S, int COLL, bool LES, bool SR = false, bool ONCE = false, class Addr>
 __device__ __forceinline__ void step_node_at(const StepArgs<S>& a, const Addr& ad, int x, int y,
                                              int z, bool faces) {
   using R = RealOf<S>;
@@ -676,7 +692,7 @@ __device__ __forceinline__ void step_node_at(const StepArgs<S>& a, const Addr& a
   // 323, 362, 464, 495, 1105)
   if (has_struct(a.g) && struct_class(a.g, x, y, z) == kSolidStruct) return;
   R f[Q];
-  pull<S>(f, a, ad, x, y, z, faces);
+  pull<S, ONCE>(f, a, ad, x, y, z, faces);
   finish_node<S, COLL, LES, SR>(f, a, ad, x, y, z);
 }
 
@@ -695,15 +711,15 @@ __device__ __forceinline__ void step_node(const StepArgs<S>& a, int x, int y, in
 }
 
 // The fused step.  grid = flat_grid, one thread per node.
-template <class S, int COLL, bool LES, bool SR = false>
+template <class S, int COLL, bool LES, bool SR = false, bool ONCE = false>
 __global__ void __launch_bounds__(128) k_step(const __grid_constant__ StepArgs<S> a) {
   chain_wait();
   bump_step_counter<SR>(a);
   const FlatItem i = flat_item(a);
   const bool faces = __any_sync(0xffffffffu, i.face_row | (i.x == 0) | (i.x == a.g.nx - 1));
   if (!i.in) return;
-  step_node_at<S, COLL, LES, SR>(a, PlaneAddr<S>(a, i.x + a.g.px * (i.z + a.g.nz * i.y)), i.x, i.y,
-                                 i.z, faces);
+  step_node_at<S, COLL, LES, SR, ONCE>(a, PlaneAddr<S>(a, i.x + a.g.px * (i.z + a.g.nz * i.y)), i.x,
+                                       i.y, i.z, faces);
 }
 
 // ------------------------------------------------------------------ //
