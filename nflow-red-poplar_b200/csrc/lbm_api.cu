@@ -247,11 +247,7 @@ int lbm_set_solid_mask(lbm_domain* d, const unsigned char* mask) {
   // the domain restarts, so its rows can change with its step kernel
   d->g.rows = domain_rows(d);
   // the step kernel and its captured graphs depend on the geometry
-  for (int i = 0; i < 2; ++i)
-    if (d->chunk[i]) {
-      cudaGraphExecDestroy(d->chunk[i]);
-      d->chunk[i] = nullptr;
-    }
+  drop_graphs(d);
   return domain_launch_init(d, d->stream);
 }
 

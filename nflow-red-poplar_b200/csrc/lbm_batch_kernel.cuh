@@ -224,7 +224,8 @@ static_assert(sizeof(FlatSet<__half>) == sizeof(FlatSet<float>) &&
               "the host fills every format's FlatSet through the FP32 layout");
 
 template <class S, int COLL, bool LES, int MODE>
-__global__ void __launch_bounds__(kFlatBlock, 8)
+__global__ void __launch_bounds__(kFlatBlock,
+                                  MODE == kModePaired ? LBM_PAIRED_THREADS_PER_SM / kFlatBlock : 8)
     k_batch_flat(const __grid_constant__ FlatSet<S> p) {
   int s = 0;
   for (int k = 1; k < p.n; ++k) s += blockIdx.x >= p.cta_off[k];

@@ -58,8 +58,14 @@ struct lbm_domain {
   float scale = 1.f, inv_scale = 1.f;
   size_t bytes = 0;
   bool pooled = false;  // buffers belong to a batch pool (lbm_batch), not freed here
-  // CUDA graphs of kGraphSteps plain steps, one per starting lattice
+  // CUDA graphs, one per starting lattice (AA: layout): kGraphSteps plain
+  // steps, and the last rest_steps steps of a run (issue_run)
   cudaGraphExec_t chunk[2] = {nullptr, nullptr};
+  cudaGraphExec_t rest[2] = {nullptr, nullptr};
+  int rest_steps[2] = {0, 0};
+  int rest_seen[2] = {0, 0};  // length of the last rest launched step by step
+  int rest_times[2] = {0, 0}; // ... and how many times in a row
+  int runs = 0;               // runs issued
   cudaStream_t capture = nullptr;
   // snapshot of the macroscopic state for the output writers
   // (lbm_snapshot / lbm_save_snapshot)
@@ -234,6 +240,10 @@ inline dim3 flat_grid(const Geometry& g) {
   return dim3((unsigned)((plane + kFlat - 1) / kFlat), g.ny, 1);
 }
 
+// lattices up to this size are run through forwards and backwards in turn
+// (flat_item)
+constexpr long long kTurnBytes = 400ll << 20;
+
 template <class S>
 StepArgs<S> make_args(const lbm_domain* d, const void* src, void* dst, long long k) {
   using R = RealOf<S>;
@@ -251,7 +261,7 @@ StepArgs<S> make_args(const lbm_domain* d, const void* src, void* dst, long long
   }
   a.g = d->g;
   a.ri = row_items(d->g);
-  a.rev = src && src == d->lat[1];
+  a.rev = src && src == d->lat[1] && 2 * Q * d->qs * (long long)sizeof(S) <= kTurnBytes;
   a.mrow = ~0ull / (unsigned long long)a.ri + 1;
   a.tau = R(d->in.m_dTau);
   const double cs = (double)d->in.m_dSmagorinsky;
@@ -308,7 +318,7 @@ StepArgs<S> aa_args(const lbm_domain* d, long long k, bool den, int neighbor) {
   }
   if (den) a.den_out = d->den[(k - 1) & 1];
   a.aa_step = 1 + neighbor;
-  a.rev = neighbor;
+  a.rev = neighbor && Q * d->qs * (long long)sizeof(S) <= kTurnBytes;
   return a;
 }
 
@@ -487,6 +497,16 @@ inline int ensure_staging(lbm_domain* d, size_t bytes) {
   return LBM_OK;
 }
 
+// forget the captured steps of d
+inline void drop_graphs(lbm_domain* d) {
+  for (int i = 0; i < 2; ++i) {
+    if (d->chunk[i]) cudaGraphExecDestroy(d->chunk[i]);
+    if (d->rest[i]) cudaGraphExecDestroy(d->rest[i]);
+    d->chunk[i] = d->rest[i] = nullptr;
+    d->rest_steps[i] = d->rest_seen[i] = d->rest_times[i] = 0;
+  }
+}
+
 inline void free_all(lbm_domain* d) {
   if (!d->pooled)
   for (int i = 0; i < 2; ++i) {
@@ -513,8 +533,7 @@ inline void free_all(lbm_domain* d) {
   if (d->flag && !d->pooled) cudaFree(d->flag);  // batch members: from the pool
   if (d->partial) cudaFree(d->partial);
   if (d->dout) cudaFree(d->dout);
-  for (int i = 0; i < 2; ++i)
-    if (d->chunk[i]) cudaGraphExecDestroy(d->chunk[i]);
+  drop_graphs(d);
   if (d->capture) cudaStreamDestroy(d->capture);
   if (d->ev0) cudaEventDestroy(d->ev0);
   if (d->ev1) cudaEventDestroy(d->ev1);

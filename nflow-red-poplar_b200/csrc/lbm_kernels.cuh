@@ -247,7 +247,8 @@ struct FlatItem {
 // a.rev: every other step runs through the box backwards, so that it begins
 // with the planes that the step before wrote last, which are still in the 126
 // MB L2 (forwards, a lattice larger than L2 evicts each plane before its next
-// use).  us a step forwards -> alternating: FP32 in place 112^3 35.9 -> 28.8,
+// use).  Up to kTurnBytes of lattices: beyond, what is left in the L2 is a few
+// per cent of a step, and domains stepped side by side lose that and 1 % more.  us a step forwards -> alternating: FP32 in place 112^3 35.9 -> 28.8,
 // 128^3 55 -> 46, 160^3 105 -> 96, 256^3 413 -> 408; FP32 pull 128^3 51.7 -> 50.3;
 // FP64 pull 80^3 26.4 -> 22.6, 256^3 765 -> 756; FP16 pull 160^3 79 -> 74; FP16 in
 // place 160^3 68 -> 61.  (Fetching the source of a pull step with an evict-first
@@ -274,12 +275,13 @@ __device__ __forceinline__ RealOf<S> ld(const S* p, int, float inv_scale) {
 
 // The same from the source lattice of a pull step (ONCE: fetched as streaming
 // data).  The source is dead once read, so marking it lets the L2 keep what
-// the step writes for the next one, as long as one lattice about fits there:
-// us a step without -> with, FP32 80^3 11.1 -> 10.7, 96^3 21.3 -> 19.6, 128^3 (160 MB)
-// 50.2 -> 49.7; FP64 80^3 22.6 -> 20.6, 96^3 40.1 -> 38.5.  Beyond, a sector that two
-// warps share is gone before the second reads it: FP32 160^3 (311 MB) 99 -> 102,
-// 256^3 396 -> 417; the 16-bit kernels only lose (FP16 128^3 37.0 -> 39.9).
-constexpr long long kOnceBytes = 160ll << 20;  // largest lattice fetched that way
+// the step writes for the next one.  Three 64^3 FP32 SRT boxes (20 MB a lattice)
+// stepped at the same time: 565 us for 100 steps of one, 484 with the mark; one
+// alone the same either way.  Larger lattices win alone (96^3 FP32 21.3 -> 19.5
+// us a step) and lose beside others (three 180x60x68, 56 MB: 1376 -> 1666 us), as
+// a sector that two warps share is gone before the second reads it; the
+// 16-bit kernels only lose.
+constexpr long long kOnceBytes = 32ll << 20;  // largest lattice fetched that way
 template <class S, bool ONCE>
 __device__ __forceinline__ RealOf<S> ld_src(const S* p, int q, float inv_scale) {
   if constexpr (ONCE)
@@ -1328,19 +1330,17 @@ __host__ __device__ __forceinline__ bool paired_kernel_applies(const Geometry& g
   return !has_struct(g) && (g.px >> 1) <= g.nx - 2;
 }
 
-// Resident threads per SM the register budget is sized for: 1024 (64
-// registers per thread) measured fastest on the 256^3 cavity (55k MLUPS
-// against 48k at 768 and 50k at 896; more warps hide more load latency,
-// which outweighs the few spilled registers).
+// Resident threads per SM the register budget is sized for: 768 (80 registers,
+// no spills).  us a step at 640 / 768 / 896 / 1024: 48^3 5.0 / 4.9 / 5.8 / 6.6, 96^3
+// 17.7 / 17.8 / 17.4 / 17.6, 200x104x96 37.8 / 37.4 / 36.6 / 37.0, 256^3 302 / 293 /
+// 291 / 297: short steps wait for the spilled registers of their face words,
+// which is more than what the extra warps hide in long ones.
 #ifndef LBM_PAIRED_THREADS_PER_SM
-#define LBM_PAIRED_THREADS_PER_SM 1024
+#define LBM_PAIRED_THREADS_PER_SM 768
 #endif
 
 // grid = flat_grid, one word (two nodes) per thread; a.srcd[q] = plane q minus
 // the donor offset 2 c_x + px (c_z + nz c_y)
-#ifndef LBM_PAIRED_SR_THREADS_PER_SM
-#define LBM_PAIRED_SR_THREADS_PER_SM 768
-#endif
 // One word w (0 <= w < px/2) of row (y, z): the step of its two nodes
 // (shared by the single-domain and batched kernels).  faces: some lane of the
 // caller's warp is in a row on a y or z face (that row at least must pass it).
@@ -1459,8 +1459,7 @@ __device__ __forceinline__ void paired_word(const StepArgs<S>& a, int w, int y, 
 }
 
 template <class S, int COLL, bool LES, bool SR>
-__global__ void __launch_bounds__(128, (SR ? LBM_PAIRED_SR_THREADS_PER_SM
-                                           : LBM_PAIRED_THREADS_PER_SM) / 128)
+__global__ void __launch_bounds__(128, LBM_PAIRED_THREADS_PER_SM / 128)
     k_step_paired(const __grid_constant__ StepArgs<S> a) {
   chain_wait();
   bump_step_counter<SR>(a);

@@ -36,13 +36,86 @@ int ops_launch_init(lbm_domain* d, cudaStream_t st) {
   });
 }
 
+// Capture what emit(stream) launches into *g, unless it is there already.
+template <class Emit>
+int capture_graph(lbm_domain* d, cudaGraphExec_t* g, Emit&& emit) {
+  if (*g) return LBM_OK;
+  if (!d->capture) CK(cudaStreamCreateWithFlags(&d->capture, cudaStreamNonBlocking));
+  CK(cudaStreamBeginCapture(d->capture, cudaStreamCaptureModeThreadLocal));
+  emit(d->capture);
+  cudaGraph_t graph;
+  CK(cudaStreamEndCapture(d->capture, &graph));
+  const cudaError_t e = cudaGraphInstantiate(g, graph, 0);
+  cudaGraphDestroy(graph);
+  if (e != cudaSuccess)
+    return set_error(LBM_ERR_CUDA, "graph instantiation failed: %s", cudaGetErrorString(e));
+  return LBM_OK;
+}
+
+// Issue n steps from the state (d->cur, d->step), which they leave advanced:
+// chunk(stream, cur, k) launches kGraphSteps plain steps after step k,
+// rest(stream, m, cur, k) the last m steps of a run with their outputs.
+//
+// Launched one by one a step costs the host 2 to 3 us, which is more than the
+// GPU needs for a box below about 48^3 (or a third of a 64^3 one when several
+// are stepped side by side), so the steps are launched as CUDA graphs, which
+// cost one launch.  Building one costs as much as some 40 launches: the chunk
+// is built for a run of at least kLongRun chunks or a domain that has run
+// before, the rest once two runs from the same lattice have ended in rests of
+// the same length (ten in a row to replace one), so that a single short run
+// pays for neither.  On a stream
+// that is being captured the steps are launched one by one (into that graph).
+constexpr int kLongRun = 8;
+constexpr int kShortestRest = 4;
+constexpr int kRestFirst = 1, kRestReplace = 9;  // equal rests before a graph
+template <class Chunk, class Rest>
+int issue_run(lbm_domain* d, int n, Chunk&& chunk, Rest&& rest) {
+  const int full = n > 2 ? (n - 2) / kGraphSteps : 0, m = n - full * kGraphSteps;
+  const int cur = d->cur;  // a chunk has an even number of steps
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  CK(cudaStreamIsCapturing(d->stream, &cs));
+  const bool graphs = cs == cudaStreamCaptureStatusNone;
+  int rc;
+  if (graphs && full > 0 && (full >= kLongRun || d->runs > 0)) {
+    const long long k = d->step;
+    if ((rc = capture_graph(d, &d->chunk[cur], [&](cudaStream_t st) { chunk(st, cur, k); })))
+      return rc;
+    for (int i = 0; i < full; ++i) CK(cudaGraphLaunch(d->chunk[cur], d->stream));
+  } else {
+    for (int i = 0; i < full; ++i) chunk(d->stream, cur, d->step + (long long)i * kGraphSteps);
+  }
+  const long long k = d->step + (long long)full * kGraphSteps;
+  if (graphs && m >= kShortestRest && d->rest[cur] && d->rest_steps[cur] == m) {
+    CK(cudaGraphLaunch(d->rest[cur], d->stream));
+  } else if (graphs && m >= kShortestRest && d->rest_seen[cur] == m &&
+             d->rest_times[cur] >= (d->rest[cur] ? kRestReplace : kRestFirst)) {
+    if (d->rest[cur]) {
+      CK(cudaGraphExecDestroy(d->rest[cur]));  // freed when its last launch is done
+      d->rest[cur] = nullptr;
+    }
+    if ((rc = capture_graph(d, &d->rest[cur], [&](cudaStream_t st) { rest(st, m, cur, k); })))
+      return rc;
+    d->rest_steps[cur] = m;
+    CK(cudaGraphLaunch(d->rest[cur], d->stream));
+  } else {
+    rest(d->stream, m, cur, k);
+    d->rest_times[cur] = d->rest_seen[cur] == m ? d->rest_times[cur] + 1 : 1;
+    d->rest_seen[cur] = m;
+  }
+  ++d->runs;
+  d->step += n;
+  d->cur ^= n & 1;
+  d->post_direct = false;
+  CK(cudaGetLastError());
+  return LBM_OK;
+}
+
 template <class S>
 int ops_run_pull(lbm_domain* d, int nsteps) {
   return with_model<S>(d, [&](auto coll, auto les) -> int {
     constexpr int C = decltype(coll)::value;
     constexpr bool L = decltype(les)::value;
-    // one plain step (no side outputs unless requested)
-    auto step_args = [&](long long k, bool den, bool vel, int cur) {
+    auto launch = [&](cudaStream_t st, int cur, long long k, bool den, bool vel) {
       StepArgs<S> a = make_args<S>(d, d->lat[cur], d->lat[cur ^ 1], k);
       if (den) a.den_out = d->den[k & 1];
       if (vel) {
@@ -50,82 +123,54 @@ int ops_run_pull(lbm_domain* d, int nsteps) {
         a.uy_out = d->uy;
         a.uz_out = d->uz;
       }
-      return a;
+      launch_step<S, C, L>(d, a, st);
     };
-    int plain = nsteps > 2 ? nsteps - 2 : 0;  // the last two steps write rho / u
-    // whole graph chunks of kGraphSteps plain steps
-    if (plain >= 2 * kGraphSteps) {
-      cudaGraphExec_t& g = d->chunk[d->cur];
-      if (!g) {
-        if (!d->capture) CK(cudaStreamCreateWithFlags(&d->capture, cudaStreamNonBlocking));
-        CK(cudaStreamBeginCapture(d->capture, cudaStreamCaptureModeThreadLocal));
-        int cur = d->cur;
-        long long k = d->step;
-        for (int i = 0; i < kGraphSteps; ++i) {
-          ++k;
-          launch_step<S, C, L>(d, step_args(k, false, false, cur), d->capture);
-          cur ^= 1;
-        }
-        cudaGraph_t graph;
-        CK(cudaStreamEndCapture(d->capture, &graph));
-        cudaError_t e = cudaGraphInstantiate(&g, graph, 0);
-        cudaGraphDestroy(graph);
-        if (e != cudaSuccess)
-          return set_error(LBM_ERR_CUDA, "graph instantiation failed: %s",
-                           cudaGetErrorString(e));
-      }
-      while (plain >= kGraphSteps) {
-        CK(cudaGraphLaunch(g, d->stream));
-        d->step += kGraphSteps;  // even: cur and plane parity unchanged
-        plain -= kGraphSteps;
-      }
-    }
-    const int rest = plain + (nsteps > 2 ? 2 : nsteps);
-    for (int i = 0; i < rest; ++i) {
-      const long long k = d->step + 1;
-      launch_step<S, C, L>(d, step_args(k, i >= rest - 2, i == rest - 1, d->cur), d->stream);
-      d->cur ^= 1;
-      d->step = k;
-    }
-    d->post_direct = false;
-    CK(cudaGetLastError());
-    return LBM_OK;
+    return issue_run(
+        d, nsteps,
+        [&](cudaStream_t st, int cur, long long k) {
+          for (int i = 0; i < kGraphSteps; ++i) launch(st, cur ^ (i & 1), k + 1 + i, false, false);
+        },
+        // the last two steps write rho, the last one u
+        [&](cudaStream_t st, int m, int cur, long long k) {
+          for (int i = 0; i < m; ++i)
+            launch(st, cur ^ (i & 1), k + 1 + i, i >= m - 2, i == m - 1);
+        });
   });
 }
 
-// nsteps AA steps (local and neighbour steps alternate with the layout),
-// in graph chunks where possible; the last two steps write the rho of their
-// input arF (the previous-step density of the residual), then k_aa_macro
-// writes rho and u of the final arF.
-// rho and u of the AA state after step d->step into den[step & 1] and u,
-// from either layout; the face buffers are those of AA step s (k = s + 1)
+// rho and u of the AA state after step `step` (layout cur) into den[step & 1]
+// and u; the face buffers are those of AA step s (k = s + 1)
 template <class S>
-int ops_aa_macro(lbm_domain* d) {
-  StepArgs<S> m = aa_args<S>(d, d->step + 1, false, d->cur);
-  m.den_out = d->den[d->step & 1];
+int aa_macro_on(lbm_domain* d, cudaStream_t st, int cur, long long step, int entry) {
+  StepArgs<S> m = aa_args<S>(d, step + 1, false, cur);
+  m.den_out = d->den[step & 1];
   m.ux_out = d->ux;
   m.uy_out = d->uy;
   m.uz_out = d->uz;
-  const int entry = d->post_direct ? kAAComplete : kAAPending;
   const dim3 bf(kFlat);
   if constexpr (kDev<S>) {
     if (d->g.rows == kRowsQuad) {
-      if (d->cur)
+      if (cur)
         launch_chained(k_aa_words<S, COLL_SRT, false, false, 1, true>, aa_neighbor_grid(d->g), bf,
-                       d->stream, m, entry);
+                       st, m, entry);
       else
-        launch_chained(k_aa_words<S, COLL_SRT, false, false, 0, true>, flat_grid(d->g), bf,
-                       d->stream, m, entry);
+        launch_chained(k_aa_words<S, COLL_SRT, false, false, 0, true>, flat_grid(d->g), bf, st, m,
+                       entry);
       CK(cudaGetLastError());
       return LBM_OK;
     }
   }
-  if (d->cur)
-    launch_chained(k_aa_macro<S, 1>, flat_grid(d->g), bf, d->stream, m, entry);
+  if (cur)
+    launch_chained(k_aa_macro<S, 1>, flat_grid(d->g), bf, st, m, entry);
   else
-    launch_chained(k_aa_macro<S, 0>, flat_grid(d->g), bf, d->stream, m, entry);
+    launch_chained(k_aa_macro<S, 0>, flat_grid(d->g), bf, st, m, entry);
   CK(cudaGetLastError());
   return LBM_OK;
+}
+
+template <class S>
+int ops_aa_macro(lbm_domain* d) {
+  return aa_macro_on<S>(d, d->stream, d->cur, d->step, d->post_direct ? kAAComplete : kAAPending);
 }
 
 template <class S>
@@ -181,55 +226,36 @@ int ops_run_aa(lbm_domain* d, int nsteps) {
       else
         launch_chained(k_aa_step<S, C, L, 0>, ga, bf, st, a, entry);
     };
-    auto one = [&](bool den) {
-      const long long k = d->step + 1;
-      const int entry = d->aa_first ? kAAFromInit : (d->post_direct ? kAAComplete : kAAPending);
-      launch(d->stream, args(k, den, d->cur), d->cur, entry);
-      d->aa_first = false;
-      d->post_direct = false;
-      d->cur ^= 1;
-      d->step = k;
-    };
-    int left = nsteps;
     // the first step from a complete natural layout (initial state, import)
     // has its own entry mode: never inside a graph
-    if ((d->aa_first || d->post_direct) && left > 0) {
-      one(left <= 2);
-      --left;
+    int left = nsteps;
+    if (d->aa_first || d->post_direct) {
+      launch(d->stream, args(d->step + 1, left <= 2, 0), 0, d->aa_first ? kAAFromInit : kAAComplete);
+      d->aa_first = false;
+      d->post_direct = false;
+      d->cur = 1;
+      ++d->step;
+      if (--left == 0) return ops_aa_macro<S>(d);
     }
-    int plain = left > 2 ? left - 2 : 0;
-    if (plain >= 2 * kGraphSteps) {
-      cudaGraphExec_t& g = d->chunk[d->cur];
-      if (!g) {
-        if (!d->capture) CK(cudaStreamCreateWithFlags(&d->capture, cudaStreamNonBlocking));
-        CK(cudaStreamBeginCapture(d->capture, cudaStreamCaptureModeThreadLocal));
-        int cur = d->cur;
-        long long k = d->step;
-        for (int i = 0; i < kGraphSteps; ++i) {
-          ++k;
-          launch(d->capture, args(k, false, cur), cur, kAAPending);
-          cur ^= 1;
-        }
-        cudaGraph_t graph;
-        CK(cudaStreamEndCapture(d->capture, &graph));
-        cudaError_t e = cudaGraphInstantiate(&g, graph, 0);
-        cudaGraphDestroy(graph);
-        if (e != cudaSuccess)
-          return set_error(LBM_ERR_CUDA, "graph instantiation failed: %s",
-                           cudaGetErrorString(e));
-      }
-      while (plain >= kGraphSteps) {
-        CK(cudaGraphLaunch(g, d->stream));
-        d->step += kGraphSteps;  // even: the layout is unchanged
-        plain -= kGraphSteps;
-        left -= kGraphSteps;
-      }
-    }
-    while (left > 0) {
-      one(left <= 2);
-      --left;
-    }
-    return ops_aa_macro<S>(d);
+    int rc = LBM_OK;
+    const int irc = issue_run(
+        d, left,
+        [&](cudaStream_t st, int cur, long long k) {
+          for (int i = 0; i < kGraphSteps; ++i) {
+            const int nb = cur ^ (i & 1);
+            launch(st, args(k + 1 + i, false, nb), nb, kAAPending);
+          }
+        },
+        // the last two steps write the rho of their input arF (the previous-step
+        // density of the residual), then rho and u of the final arF
+        [&](cudaStream_t st, int m, int cur, long long k) {
+          for (int i = 0; i < m; ++i) {
+            const int nb = cur ^ (i & 1);
+            launch(st, args(k + 1 + i, i >= m - 2, nb), nb, kAAPending);
+          }
+          rc = aa_macro_on<S>(d, st, cur ^ (m & 1), k + m, kAAPending);
+        });
+    return irc ? irc : rc;
   });
 }
 

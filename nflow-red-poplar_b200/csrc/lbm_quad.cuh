@@ -299,12 +299,13 @@ __global__ void __launch_bounds__(128, LBM_QUAD_THREADS_PER_SM / 128)
     const FlatItem i = flat_item(a);
     if (i.in) aa_word<S, COLL, LES, SR, 0, false, MACRO>(a, i.x, i.y, i.z, entry);
   } else if ((int)blockIdx.y < a.g.ny - 2) {
-    // backwards, as flat_item with a.rev: the local steps run forwards
-    const unsigned t = (gridDim.x - 1 - blockIdx.x) * 128u + threadIdx.x;
+    // backwards with a.rev, as flat_item
+    const unsigned t = (a.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * 128u + threadIdx.x;
     const int r = (int)fastdiv(t, a.mrow);
     if (r < a.g.nz - 2)
-      aa_word<S, COLL, LES, SR, 1, false, MACRO>(a, (int)t - r * a.ri,
-                                                 a.g.ny - 2 - (int)blockIdx.y, r + 1, entry);
+      aa_word<S, COLL, LES, SR, 1, false, MACRO>(
+          a, (int)t - r * a.ri, a.rev ? a.g.ny - 2 - (int)blockIdx.y : 1 + (int)blockIdx.y, r + 1,
+          entry);
   } else {
     const unsigned c = (blockIdx.y - (unsigned)(a.g.ny - 2)) * gridDim.x + blockIdx.x;
     const unsigned t = c * 128u + threadIdx.x;
