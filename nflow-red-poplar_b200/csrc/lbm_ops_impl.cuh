@@ -59,14 +59,14 @@ int capture_graph(lbm_domain* d, cudaGraphExec_t* g, Emit&& emit) {
 // Launched one by one a step costs the host 2 to 3 us, which is more than the
 // GPU needs for a box below about 48^3 (or a third of a 64^3 one when several
 // are stepped side by side), so the steps are launched as CUDA graphs, which
-// cost one launch.  Building one costs as much as some 40 launches: the chunk
+// cost one launch (even a single step: 16^3 FP32 pull, three side by side, one
+// step a run 7.6 us -> 6.2, three steps 14.4 -> 6.5).  Building one costs as much as some 40 launches: the chunk
 // is built for a run of at least kLongRun chunks or a domain that has run
 // before, the rest once two runs from the same lattice have ended in rests of
 // the same length (ten in a row to replace one), so that a single short run
 // pays for neither.  On a stream
 // that is being captured the steps are launched one by one (into that graph).
 constexpr int kLongRun = 8;
-constexpr int kShortestRest = 4;
 constexpr int kRestFirst = 1, kRestReplace = 9;  // equal rests before a graph
 template <class Chunk, class Rest>
 int issue_run(lbm_domain* d, int n, Chunk&& chunk, Rest&& rest) {
@@ -85,9 +85,9 @@ int issue_run(lbm_domain* d, int n, Chunk&& chunk, Rest&& rest) {
     for (int i = 0; i < full; ++i) chunk(d->stream, cur, d->step + (long long)i * kGraphSteps);
   }
   const long long k = d->step + (long long)full * kGraphSteps;
-  if (graphs && m >= kShortestRest && d->rest[cur] && d->rest_steps[cur] == m) {
+  if (graphs && d->rest[cur] && d->rest_steps[cur] == m) {
     CK(cudaGraphLaunch(d->rest[cur], d->stream));
-  } else if (graphs && m >= kShortestRest && d->rest_seen[cur] == m &&
+  } else if (graphs && d->rest_seen[cur] == m &&
              d->rest_times[cur] >= (d->rest[cur] ? kRestReplace : kRestFirst)) {
     if (d->rest[cur]) {
       CK(cudaGraphExecDestroy(d->rest[cur]));  // freed when its last launch is done
