@@ -491,7 +491,14 @@ int issue_chunk_flat(lbm_batch* b, int steps_offered, long long* lups) {
         kp.blockDim = dim3(kFlatBlock);
       }
       cudaGraphNode_t node;
-      e = cudaGraphAddKernelNode(&node, gr, prev ? &prev : nullptr, prev ? 1 : 0, &kp);
+      e = cudaGraphAddKernelNode(&node, gr, nullptr, 0, &kp);
+      if (prev && e == cudaSuccess) {
+        cudaGraphEdgeData edge;
+        std::memset(&edge, 0, sizeof(edge));
+        edge.from_port = cudaGraphKernelNodePortProgrammatic;
+        edge.type = cudaGraphDependencyTypeProgrammatic;
+        e = cudaGraphAddDependencies_v2(gr, &prev, &node, &edge, 1);
+      }
       prev = node;
     }
   }

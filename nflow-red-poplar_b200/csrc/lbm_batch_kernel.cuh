@@ -193,8 +193,10 @@ __global__ void __launch_bounds__(256, MINB) k_batch_step(const BatchTables* __r
 // that depends on blockIdx and parameters only, so it is the same for every
 // thread, and the member's arguments read from the parameter space like
 // those of a single-domain kernel.  Each set is a chain of launches in the
-// chunk graph, independent of the other sets, so the sets' launches overlap
-// on the GPU and fill each other's tails.  A set of one member launches the
+// chunk graph (programmatic edges: the next launch's CTAs are placed while the
+// one ahead drains, 64 FP32 32^3 members 69.8 -> 66.2 us a step), independent of
+// the other sets, so the sets' launches overlap on the GPU and fill each
+// other's tails.  A set of one member launches the
 // member's single-domain step kernel instead (its arguments are kernel
 // parameters there as well).
 // ------------------------------------------------------------------ //
@@ -223,10 +225,14 @@ static_assert(sizeof(FlatSet<__half>) == sizeof(FlatSet<float>) &&
                   sizeof(StepArgs<__nv_bfloat16>) == sizeof(StepArgs<float>),
               "the host fills every format's FlatSet through the FP32 layout");
 
+// Resident CTAs: 8 (64 registers).  Paired words and the face forms of the AA
+// step spill a few, which the other members hide: 16 FP16 64^3 members 90 us a
+// step against 97 with 80 registers, 64 FP32 in-place 32^3 members 75 against 82
+// with 72.
 template <class S, int COLL, bool LES, int MODE>
-__global__ void __launch_bounds__(kFlatBlock,
-                                  MODE == kModePaired ? LBM_PAIRED_THREADS_PER_SM / kFlatBlock : 8)
+__global__ void __launch_bounds__(kFlatBlock, 8)
     k_batch_flat(const __grid_constant__ FlatSet<S> p) {
+  chain_wait();
   int s = 0;
   for (int k = 1; k < p.n; ++k) s += blockIdx.x >= p.cta_off[k];
   const StepArgs<S>& a = p.args[s];
