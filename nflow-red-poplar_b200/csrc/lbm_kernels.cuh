@@ -328,6 +328,37 @@ struct RowAddr {
   __device__ __forceinline__ float scale() const { return a.scale; }
 };
 
+// keBoundaryInlet: ftemp[d] - 6.0 w_d rho(x+1) (c_d . u_in), FP64 literal
+template <class S, int q>
+__device__ __forceinline__ RealOf<S> inlet_value(RealOf<S> fo, float rho, RealOf<S> eu) {
+  using R = RealOf<S>;
+  return R((double)fo - 6.0 * (double)weight<R>(opp(q)) * (double)rho * (double)eu);
+}
+// keBoundaryOutlet: anti-bounce-back at RefDen with u extrapolated from the
+// node and its inner neighbour of the previous step
+template <class S>
+__device__ __forceinline__ void outlet_velocity(const StepArgs<S>& a, int yz, RealOf<S> (&b)[3]) {
+  const int P = a.g.ny * a.g.nz;
+  const float* u0 = a.pu_in;          // x = nx-1
+  const float* u1 = a.pu_in + 3 * P;  // x = nx-2
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    b[i] = RealOf<S>((double)u0[i * P + yz] + 0.5 * (double)(u0[i * P + yz] - u1[i * P + yz]));
+}
+template <class S, int q>
+__device__ __forceinline__ RealOf<S> outlet_value(const StepArgs<S>& a, RealOf<S> fo,
+                                                  const RealOf<S> (&b)[3]) {
+  using R = RealOf<S>;
+  constexpr int d = opp(q);
+  const R usq = b[0] * b[0] + b[1] * b[1] + b[2] * b[2];
+  const R eu = R(cx(d)) * b[0] + R(cy(d)) * b[1] + R(cz(d)) * b[2];
+  const double v = -(double)fo + 2.0 * (double)weight<R>(d) * (double)a.rho0 *
+                                     (1.0 + 4.5 * ((double)eu * (double)eu) - 1.5 * (double)usq);
+  // deviations: g_q = f_q - w = -(g_d + w) + X - w (w_q = w_d)
+  if constexpr (kDev<S>) return R(v - 2.0 * (double)weight<R>(d));
+  return R(v);
+}
+
 // Boundary value of population q at a node whose donor x - c_q is outside
 // the domain.  d = opp(q) is the reference's "outside" direction; fo is
 // f*_{k-1}[d] at the node itself (arFTemp[d](x) in the reference).
@@ -355,25 +386,14 @@ __device__ __forceinline__ RealOf<S> boundary_value(const StepArgs<S>& a, int t,
       eu = add_rn(add_rn(mul_rn(R(cx(d)), a.ulx), mul_rn(R(cy(d)), a.uly)),
                   mul_rn(R(cz(d)), a.ulz));
     }
-    const double v = (double)fo - 6.0 * (double)weight<R>(d) * (double)a.prho_in[yz] * (double)eu;
-    return R(v);
+    return inlet_value<S, q>(fo, a.prho_in[yz], eu);
   }
   if (t == NODE_OUTLET) {
     // keBoundaryOutlet: anti-bounce-back at RefDen with u extrapolated
     // from the node and its inner neighbour of the previous step
-    const int P = a.g.ny * a.g.nz;
-    const float* u0 = a.pu_in;          // x = nx-1
-    const float* u1 = a.pu_in + 3 * P;  // x = nx-2
-    const R bx = R((double)u0[yz] + 0.5 * (double)(u0[yz] - u1[yz]));
-    const R by = R((double)u0[P + yz] + 0.5 * (double)(u0[P + yz] - u1[P + yz]));
-    const R bz = R((double)u0[2 * P + yz] + 0.5 * (double)(u0[2 * P + yz] - u1[2 * P + yz]));
-    const R usq = bx * bx + by * by + bz * bz;
-    const R eu = R(cx(d)) * bx + R(cy(d)) * by + R(cz(d)) * bz;
-    const double v = -(double)fo + 2.0 * (double)weight<R>(d) * (double)a.rho0 *
-                                       (1.0 + 4.5 * ((double)eu * (double)eu) - 1.5 * (double)usq);
-    // deviations: g_q = f_q - w = -(g_d + w) + X - w (w_q = w_d)
-    if constexpr (kDev<S>) return R(v - 2.0 * (double)weight<R>(d));
-    return R(v);
+    R b[3];
+    outlet_velocity<S>(a, yz, b);
+    return outlet_value<S, q>(a, fo, b);
   }
   return fo;  // no rule for this node type: plain bounce-back
 }

@@ -184,18 +184,32 @@ __device__ __forceinline__ void aa_word(const StepArgs<S>& a, int w, int y, int 
   // f*_{opp q} there.  One lane of a row evaluates them; a kernel of its own
   // after each step, which left the values for the next one, cost a launch
   // and 10 scattered reads a row: 32^3 10.3 us a step against 4.8 here,
-  // 256x72x64 26.8 against 20.9, 512x128x128 148 against 142.5.
+  // 256x72x64 26.8 against 20.9, 512x128x128 148 against 138.
+  // What the rules read is fetched with the populations.
+  const int yz = y * a.g.nz + z;
+  const bool open_rows = !FACE && a.g.casetype == CHANNEL &&
+                         (NB || (entry == kAAPending && y > 0 && y < a.g.ny - 1 && z > 0 &&
+                                 z < a.g.nz - 1));
+  [[maybe_unused]] float in_rho = 0.0f, in_u = 0.0f;
+  [[maybe_unused]] float out_u[3] = {0.0f, 0.0f, 0.0f};
+  if (open_rows) {
+    if (seam_lo) {
+      in_rho = a.prho_in[yz];
+      in_u = mul_rn(-1.0f, a.inlet_u[yz]);  // c_d . u_in, c_d,x = -1
+    }
+    if (seam_hi) outlet_velocity<S>(a, yz, out_u);
+  }
   auto open_face_rules = [&](F2 (&f)[Q], int hb) {
     if (hb == 0 && seam_lo) {
       static_for<0, Q>([&](auto qc) {
         constexpr int q = decltype(qc)::value;
-        if constexpr (cx(q) == 1) f[q].v.x = boundary_value<S, q>(a, NODE_INLET, f[q].v.x, y, z);
+        if constexpr (cx(q) == 1) f[q].v.x = inlet_value<S, q>(f[q].v.x, in_rho, in_u);
       });
     }
     if (hb == 1 && seam_hi) {
       static_for<0, Q>([&](auto qc) {
         constexpr int q = decltype(qc)::value;
-        if constexpr (cx(q) == -1) f[q].v.y = boundary_value<S, q>(a, NODE_OUTLET, f[q].v.y, y, z);
+        if constexpr (cx(q) == -1) f[q].v.y = outlet_value<S, q>(a, f[q].v.y, out_u);
       });
     }
   };
@@ -230,9 +244,7 @@ __device__ __forceinline__ void aa_word(const StepArgs<S>& a, int w, int y, int 
     } else {
       // channels: rows off the faces (neighbour step), the pending natural
       // slots of the inlet and outlet nodes (local step)
-      const bool off_face = NB || (entry == kAAPending && y > 0 && y < a.g.ny - 1 && z > 0 &&
-                                   z < a.g.nz - 1);
-      if (a.g.casetype == CHANNEL && off_face) open_face_rules(f, hb);
+      if (open_rows) open_face_rules(f, hb);
     }
     PairState<F2> ps;
     make_pairs<F2, true>(f, ps);
