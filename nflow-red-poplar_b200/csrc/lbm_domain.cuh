@@ -241,8 +241,10 @@ inline dim3 flat_grid(const Geometry& g) {
 }
 
 // lattices up to this size are run through forwards and backwards in turn
-// (flat_item)
-constexpr long long kTurnBytes = 400ll << 20;
+// (flat_item): both of a pull domain together, the one of an in-place domain,
+// which finds twice the planes in the L2 (600 MB FP32 in place 208 -> 200 us a
+// step alone, the same beside two others)
+constexpr long long kTurnBytes = 400ll << 20, kTurnBytesAA = 800ll << 20;
 
 template <class S>
 StepArgs<S> make_args(const lbm_domain* d, const void* src, void* dst, long long k) {
@@ -318,7 +320,7 @@ StepArgs<S> aa_args(const lbm_domain* d, long long k, bool den, int neighbor) {
   }
   if (den) a.den_out = d->den[(k - 1) & 1];
   a.aa_step = 1 + neighbor;
-  a.rev = neighbor && Q * d->qs * (long long)sizeof(S) <= kTurnBytes;
+  a.rev = neighbor && Q * d->qs * (long long)sizeof(S) <= kTurnBytesAA;
   return a;
 }
 

@@ -247,7 +247,7 @@ struct FlatItem {
 // a.rev: every other step runs through the box backwards, so that it begins
 // with the planes that the step before wrote last, which are still in the 126
 // MB L2 (forwards, a lattice larger than L2 evicts each plane before its next
-// use).  Up to kTurnBytes of lattices: beyond, what is left in the L2 is a few
+// use).  Up to kTurnBytes(AA) of lattices: beyond, what is left in the L2 is a few
 // per cent of a step, and domains stepped side by side lose that and 1 % more.  us a step forwards -> alternating: FP32 in place 112^3 35.9 -> 28.8,
 // 128^3 55 -> 46, 160^3 105 -> 96, 256^3 413 -> 408; FP32 pull 128^3 51.7 -> 50.3;
 // FP64 pull 80^3 26.4 -> 22.6, 256^3 765 -> 756; FP16 pull 160^3 79 -> 74; FP16 in
