@@ -247,7 +247,7 @@ int lbm_set_solid_mask(lbm_domain* d, const unsigned char* mask) {
   // the domain restarts, so its rows can change with its step kernel
   d->g.rows = domain_rows(d);
   // the step kernel and its captured graphs depend on the geometry
-  drop_graphs(d);
+  d->graphs.drop();
   return domain_launch_init(d, d->stream);
 }
 

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "lbm_internal.h"
+#include "lbm_issue.h"
 #include "lbm_kernels.cuh"
 #include "lbm_tma.cuh"
 
@@ -58,15 +59,7 @@ struct lbm_domain {
   float scale = 1.f, inv_scale = 1.f;
   size_t bytes = 0;
   bool pooled = false;  // buffers belong to a batch pool (lbm_batch), not freed here
-  // CUDA graphs, one per starting lattice (AA: layout): kGraphSteps plain
-  // steps, and the last rest_steps steps of a run (issue_run)
-  cudaGraphExec_t chunk[2] = {nullptr, nullptr};
-  cudaGraphExec_t rest[2] = {nullptr, nullptr};
-  int rest_steps[2] = {0, 0};
-  int rest_seen[2] = {0, 0};  // length of the last rest launched step by step
-  int rest_times[2] = {0, 0}; // ... and how many times in a row
-  int runs = 0;               // runs issued
-  cudaStream_t capture = nullptr;
+  lbm::RunGraphs graphs;  // captured steps (issue_run)
   // snapshot of the macroscopic state for the output writers
   // (lbm_snapshot / lbm_save_snapshot)
   float* snap_dev = nullptr;       // [4][N] rho, ux, uy, uz on the device
@@ -81,10 +74,6 @@ struct lbm_domain {
   // aa_first: the next step is the first after the initial state
   bool aa_first = false;
 };
-
-// steps per captured graph chunk (even, so that a chunk returns the lattices
-// and the boundary planes to the parity it started from)
-constexpr int kGraphSteps = 32;
 
 namespace lbm {
 
@@ -341,7 +330,8 @@ int with_model(const lbm_domain* d, F&& f) {
 // are visible.  What this hides is the launch latency and the ramp of every
 // step: 24^3 to 256^3 2 to 5 %.
 template <class... P, class... A>
-void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A&&... args) {
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st,
+                           A&&... args) {
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
@@ -351,22 +341,19 @@ void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st
   cfg.stream = st;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
-// the fused step kernel of the domain's storage: the packed two-node kernel
-// for the FP32-arithmetic formats (unless the scalar one is requested),
-// the scalar kernel for the FP64 build
+// the fused pull step of the domain: the paired kernel over paired rows (16-bit),
+// the two-node and TMA kernels where they are asked for, else one node per
+// thread
 template <class S, int COLL, bool LES>
-void launch_step(const lbm_domain* d, const StepArgs<S>& a, cudaStream_t st) {
+cudaError_t launch_step(const lbm_domain* d, const StepArgs<S>& a, cudaStream_t st) {
+  const dim3 gf = flat_grid(d->g), bf(kFlat);
   if constexpr (kDev<S>) {
-    if (d->g.rows == kRowsPaired) {
-      if (a.sr)
-        launch_chained(k_step_paired<S, COLL, LES, true>, flat_grid(d->g), dim3(kFlat), st, a);
-      else
-        launch_chained(k_step_paired<S, COLL, LES, false>, flat_grid(d->g), dim3(kFlat), st, a);
-      return;
-    }
+    if (d->g.rows == kRowsPaired)
+      return a.sr ? launch_chained(k_step_paired<S, COLL, LES, true>, gf, bf, st, a)
+                  : launch_chained(k_step_paired<S, COLL, LES, false>, gf, bf, st, a);
   }
   if constexpr (!std::is_same<S, double>::value) {
     if (has_struct(d->g)) {
@@ -375,28 +362,23 @@ void launch_step(const lbm_domain* d, const StepArgs<S>& a, cudaStream_t st) {
       const int pairs = (d->g.nx + 1) / 2;
       const dim3 b(64, 1, 1), gr((pairs + 63) / 64, d->g.nz, d->g.ny);
       k_step2<S, COLL, LES><<<gr, b, 0, st>>>(a);
-      return;
-    }
-    else if (d->opt.kernel == LBM_KERNEL_TMA && d->tmap_ok) {
+      return cudaGetLastError();
+    } else if (d->opt.kernel == LBM_KERNEL_TMA && d->tmap_ok) {
       using Cfg = TmaCfg<S>;
       const int which = (a.src == (const S*)d->lat[0]) ? 0 : 1;
       // the wait test withholds one tile and bounds every wait to ~1 ms
       const int stall = d->opt.wait_test > 0 ? d->opt.wait_test - 1 : -1;
       k_step_tma<S, COLL, LES><<<d->tma_grid, Cfg::THREADS, Cfg::SMEM, st>>>(
           a, d->tmap[which], d->flag + 1, stall, stall >= 0 ? 1000 : kWaitIters);
-      return;
+      return cudaGetLastError();
     }
   }
   if constexpr (kDev<S>) {
-    if (a.sr) {
-      launch_chained(k_step<S, COLL, LES, true>, flat_grid(d->g), dim3(kFlat), st, a);
-      return;
-    }
+    if (a.sr) return launch_chained(k_step<S, COLL, LES, true>, gf, bf, st, a);
   } else if ((long long)Q * d->qs * (long long)sizeof(S) <= kOnceBytes) {
-    launch_chained(k_step<S, COLL, LES, false, true>, flat_grid(d->g), dim3(kFlat), st, a);
-    return;
+    return launch_chained(k_step<S, COLL, LES, false, true>, gf, bf, st, a);
   }
-  launch_chained(k_step<S, COLL, LES, false>, flat_grid(d->g), dim3(kFlat), st, a);
+  return launch_chained(k_step<S, COLL, LES, false>, gf, bf, st, a);
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
@@ -499,16 +481,6 @@ inline int ensure_staging(lbm_domain* d, size_t bytes) {
   return LBM_OK;
 }
 
-// forget the captured steps of d
-inline void drop_graphs(lbm_domain* d) {
-  for (int i = 0; i < 2; ++i) {
-    if (d->chunk[i]) cudaGraphExecDestroy(d->chunk[i]);
-    if (d->rest[i]) cudaGraphExecDestroy(d->rest[i]);
-    d->chunk[i] = d->rest[i] = nullptr;
-    d->rest_steps[i] = d->rest_seen[i] = d->rest_times[i] = 0;
-  }
-}
-
 inline void free_all(lbm_domain* d) {
   if (!d->pooled)
   for (int i = 0; i < 2; ++i) {
@@ -535,8 +507,8 @@ inline void free_all(lbm_domain* d) {
   if (d->flag && !d->pooled) cudaFree(d->flag);  // batch members: from the pool
   if (d->partial) cudaFree(d->partial);
   if (d->dout) cudaFree(d->dout);
-  drop_graphs(d);
-  if (d->capture) cudaStreamDestroy(d->capture);
+  d->graphs.drop();
+  if (d->graphs.capture) cudaStreamDestroy(d->graphs.capture);
   if (d->ev0) cudaEventDestroy(d->ev0);
   if (d->ev1) cudaEventDestroy(d->ev1);
   if (d->own) cudaStreamDestroy(d->own);

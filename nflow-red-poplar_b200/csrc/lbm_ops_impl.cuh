@@ -36,141 +36,52 @@ int ops_launch_init(lbm_domain* d, cudaStream_t st) {
   });
 }
 
-// Capture what emit(stream) launches into *g, unless it is there already.
-template <class Emit>
-int capture_graph(lbm_domain* d, cudaGraphExec_t* g, Emit&& emit) {
-  if (*g) return LBM_OK;
-  if (!d->capture) CK(cudaStreamCreateWithFlags(&d->capture, cudaStreamNonBlocking));
-  CK(cudaStreamBeginCapture(d->capture, cudaStreamCaptureModeThreadLocal));
-  emit(d->capture);
-  cudaGraph_t graph;
-  CK(cudaStreamEndCapture(d->capture, &graph));
-  const cudaError_t e = cudaGraphInstantiate(g, graph, 0);
-  cudaGraphDestroy(graph);
-  if (e != cudaSuccess)
-    return set_error(LBM_ERR_CUDA, "graph instantiation failed: %s", cudaGetErrorString(e));
-  return LBM_OK;
-}
-
-// Issue n steps from the state (d->cur, d->step), which they leave advanced:
-// chunk(stream, cur, k) launches kGraphSteps plain steps after step k,
-// rest(stream, m, cur, k) the last m steps of a run with their outputs.
-//
-// Launched one by one a step costs the host 2 to 3 us, which is more than the
-// GPU needs for a box below about 48^3 (or a third of a 64^3 one when several
-// are stepped side by side), so the steps are launched as CUDA graphs, which
-// cost one launch (even a single step: 16^3 FP32 pull, three side by side, one
-// step a run 7.6 us -> 6.2, three steps 14.4 -> 6.5).  Building one costs as much as some 40 launches: the chunk
-// is built for a run of at least kLongRun chunks or a domain that has run
-// before, the rest once two runs from the same lattice have ended in rests of
-// the same length (ten in a row to replace one), so that a single short run
-// pays for neither.  On a stream
-// that is being captured the steps are launched one by one (into that graph).
-constexpr int kLongRun = 8;
-constexpr int kRestFirst = 1, kRestReplace = 9;  // equal rests before a graph
-template <class Chunk, class Rest>
-int issue_run(lbm_domain* d, int n, Chunk&& chunk, Rest&& rest) {
-  const int full = n > 2 ? (n - 2) / kGraphSteps : 0, m = n - full * kGraphSteps;
-  const int cur = d->cur;  // a chunk has an even number of steps
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  CK(cudaStreamIsCapturing(d->stream, &cs));
-  const bool graphs = cs == cudaStreamCaptureStatusNone;
-  int rc;
-  if (graphs && full > 0 && (full >= kLongRun || d->runs > 0)) {
-    const long long k = d->step;
-    if ((rc = capture_graph(d, &d->chunk[cur], [&](cudaStream_t st) { chunk(st, cur, k); })))
-      return rc;
-    for (int i = 0; i < full; ++i) CK(cudaGraphLaunch(d->chunk[cur], d->stream));
-  } else {
-    for (int i = 0; i < full; ++i) chunk(d->stream, cur, d->step + (long long)i * kGraphSteps);
-  }
-  const long long k = d->step + (long long)full * kGraphSteps;
-  if (graphs && d->rest[cur] && d->rest_steps[cur] == m) {
-    CK(cudaGraphLaunch(d->rest[cur], d->stream));
-  } else if (graphs && d->rest_seen[cur] == m &&
-             d->rest_times[cur] >= (d->rest[cur] ? kRestReplace : kRestFirst)) {
-    if (d->rest[cur]) {
-      CK(cudaGraphExecDestroy(d->rest[cur]));  // freed when its last launch is done
-      d->rest[cur] = nullptr;
-    }
-    if ((rc = capture_graph(d, &d->rest[cur], [&](cudaStream_t st) { rest(st, m, cur, k); })))
-      return rc;
-    d->rest_steps[cur] = m;
-    CK(cudaGraphLaunch(d->rest[cur], d->stream));
-  } else {
-    rest(d->stream, m, cur, k);
-    d->rest_times[cur] = d->rest_seen[cur] == m ? d->rest_times[cur] + 1 : 1;
-    d->rest_seen[cur] = m;
-  }
-  ++d->runs;
-  d->step += n;
-  d->cur ^= n & 1;
-  d->post_direct = false;
-  CK(cudaGetLastError());
-  return LBM_OK;
-}
-
 template <class S>
 int ops_run_pull(lbm_domain* d, int nsteps) {
   return with_model<S>(d, [&](auto coll, auto les) -> int {
-    constexpr int C = decltype(coll)::value;
-    constexpr bool L = decltype(les)::value;
-    auto launch = [&](cudaStream_t st, int cur, long long k, bool den, bool vel) {
-      StepArgs<S> a = make_args<S>(d, d->lat[cur], d->lat[cur ^ 1], k);
-      if (den) a.den_out = d->den[k & 1];
-      if (vel) {
-        a.ux_out = d->ux;
-        a.uy_out = d->uy;
-        a.uz_out = d->uz;
-      }
-      launch_step<S, C, L>(d, a, st);
-    };
     return issue_run(
         d, nsteps,
-        [&](cudaStream_t st, int cur, long long k) {
-          for (int i = 0; i < kGraphSteps; ++i) launch(st, cur ^ (i & 1), k + 1 + i, false, false);
-        },
         // the last two steps write rho, the last one u
-        [&](cudaStream_t st, int m, int cur, long long k) {
-          for (int i = 0; i < m; ++i)
-            launch(st, cur ^ (i & 1), k + 1 + i, i >= m - 2, i == m - 1);
-        });
+        [&](cudaStream_t st, int cur, long long k, int left) {
+          StepArgs<S> a = make_args<S>(d, d->lat[cur], d->lat[cur ^ 1], k);
+          if (left < 2) a.den_out = d->den[k & 1];
+          if (left == 0) {
+            a.ux_out = d->ux;
+            a.uy_out = d->uy;
+            a.uz_out = d->uz;
+          }
+          return launch_step<S, decltype(coll)::value, decltype(les)::value>(d, a, st);
+        },
+        [](cudaStream_t, int, long long) { return cudaSuccess; });
   });
 }
 
 // rho and u of the AA state after step `step` (layout cur) into den[step & 1]
 // and u; the face buffers are those of AA step s (k = s + 1)
 template <class S>
-int aa_macro_on(lbm_domain* d, cudaStream_t st, int cur, long long step, int entry) {
+cudaError_t aa_macro_on(lbm_domain* d, cudaStream_t st, int cur, long long step, int entry) {
   StepArgs<S> m = aa_args<S>(d, step + 1, false, cur);
   m.den_out = d->den[step & 1];
   m.ux_out = d->ux;
   m.uy_out = d->uy;
   m.uz_out = d->uz;
-  const dim3 bf(kFlat);
+  const dim3 gf = flat_grid(d->g), bf(kFlat);
   if constexpr (kDev<S>) {
-    if (d->g.rows == kRowsQuad) {
-      if (cur)
-        launch_chained(k_aa_words<S, COLL_SRT, false, false, 1, true>, aa_neighbor_grid(d->g), bf,
-                       st, m, entry);
-      else
-        launch_chained(k_aa_words<S, COLL_SRT, false, false, 0, true>, flat_grid(d->g), bf, st, m,
-                       entry);
-      CK(cudaGetLastError());
-      return LBM_OK;
-    }
+    if (d->g.rows == kRowsQuad)
+      return cur ? launch_chained(k_aa_words<S, COLL_SRT, false, false, 1, true>,
+                                  aa_neighbor_grid(d->g), bf, st, m, entry)
+                 : launch_chained(k_aa_words<S, COLL_SRT, false, false, 0, true>, gf, bf, st, m,
+                                  entry);
   }
-  if (cur)
-    launch_chained(k_aa_macro<S, 1>, flat_grid(d->g), bf, st, m, entry);
-  else
-    launch_chained(k_aa_macro<S, 0>, flat_grid(d->g), bf, st, m, entry);
-  CK(cudaGetLastError());
-  return LBM_OK;
+  return cur ? launch_chained(k_aa_macro<S, 1>, gf, bf, st, m, entry)
+             : launch_chained(k_aa_macro<S, 0>, gf, bf, st, m, entry);
 }
 
 template <class S>
 int ops_aa_macro(lbm_domain* d) {
-  return aa_macro_on<S>(d, d->stream, d->cur, d->step, d->post_direct ? kAAComplete : kAAPending);
+  return launch_status(
+      aa_macro_on<S>(d, d->stream, d->cur, d->step, d->post_direct ? kAAComplete : kAAPending),
+      "rho and u");
 }
 
 template <class S>
@@ -197,65 +108,49 @@ int ops_run_aa(lbm_domain* d, int nsteps) {
         gn = aa_neighbor_grid(d->g);
       }
     }
-    auto launch = [&](cudaStream_t st, const StepArgs<S>& a, int nb, int entry) {
+    auto launch = [&](cudaStream_t st, const StepArgs<S>& a, int nb, int entry) -> cudaError_t {
       if constexpr (kDev<S>) {
+        if (words && entry != kAAFromInit) {
+          if (a.sr)
+            return nb ? launch_chained(k_aa_words<S, C, L, true, 1>, gn, bf, st, a, entry)
+                      : launch_chained(k_aa_words<S, C, L, true, 0>, gw, bf, st, a, entry);
+          return nb ? launch_chained(k_aa_words<S, C, L, false, 1>, gn, bf, st, a, entry)
+                    : launch_chained(k_aa_words<S, C, L, false, 0>, gw, bf, st, a, entry);
+        }
         if (words) {
-          if (entry != kAAFromInit) {
-            if (a.sr) {
-              if (nb)
-                launch_chained(k_aa_words<S, C, L, true, 1>, gn, bf, st, a, entry);
-              else
-                launch_chained(k_aa_words<S, C, L, true, 0>, gw, bf, st, a, entry);
-            } else {
-              if (nb)
-                launch_chained(k_aa_words<S, C, L, false, 1>, gn, bf, st, a, entry);
-              else
-                launch_chained(k_aa_words<S, C, L, false, 0>, gw, bf, st, a, entry);
-            }
-          } else {
-            StepArgs<S> an = a;  // one node per item
-            an.ri = d->g.px;
-            an.mrow = ~0ull / (unsigned long long)an.ri + 1;
-            launch_chained(k_aa_step<S, C, L, 0>, ga, bf, st, an, entry);
-          }
-          return;
+          StepArgs<S> an = a;  // one node per item
+          an.ri = d->g.px;
+          an.mrow = ~0ull / (unsigned long long)an.ri + 1;
+          return launch_chained(k_aa_step<S, C, L, 0>, ga, bf, st, an, entry);
         }
       }
-      if (nb)
-        launch_chained(k_aa_step<S, C, L, 1>, ga, bf, st, a, entry);
-      else
-        launch_chained(k_aa_step<S, C, L, 0>, ga, bf, st, a, entry);
+      return nb ? launch_chained(k_aa_step<S, C, L, 1>, ga, bf, st, a, entry)
+                : launch_chained(k_aa_step<S, C, L, 0>, ga, bf, st, a, entry);
     };
     // the first step from a complete natural layout (initial state, import)
     // has its own entry mode: never inside a graph
     int left = nsteps;
     if (d->aa_first || d->post_direct) {
-      launch(d->stream, args(d->step + 1, left <= 2, 0), 0, d->aa_first ? kAAFromInit : kAAComplete);
+      const int rc = launch_status(launch(d->stream, args(d->step + 1, left <= 2, 0), 0,
+                                          d->aa_first ? kAAFromInit : kAAComplete),
+                                   "a step");
+      if (rc) return rc;
       d->aa_first = false;
       d->post_direct = false;
       d->cur = 1;
       ++d->step;
       if (--left == 0) return ops_aa_macro<S>(d);
     }
-    int rc = LBM_OK;
-    const int irc = issue_run(
+    return issue_run(
         d, left,
-        [&](cudaStream_t st, int cur, long long k) {
-          for (int i = 0; i < kGraphSteps; ++i) {
-            const int nb = cur ^ (i & 1);
-            launch(st, args(k + 1 + i, false, nb), nb, kAAPending);
-          }
-        },
         // the last two steps write the rho of their input arF (the previous-step
-        // density of the residual), then rho and u of the final arF
-        [&](cudaStream_t st, int m, int cur, long long k) {
-          for (int i = 0; i < m; ++i) {
-            const int nb = cur ^ (i & 1);
-            launch(st, args(k + 1 + i, i >= m - 2, nb), nb, kAAPending);
-          }
-          rc = aa_macro_on<S>(d, st, cur ^ (m & 1), k + m, kAAPending);
+        // density of the residual); rho and u of the final arF follow
+        [&](cudaStream_t st, int cur, long long k, int todo) {
+          return launch(st, args(k, todo < 2, cur), cur, kAAPending);
+        },
+        [&](cudaStream_t st, int cur, long long k) {
+          return aa_macro_on<S>(d, st, cur, k, kAAPending);
         });
-    return irc ? irc : rc;
   });
 }
 
