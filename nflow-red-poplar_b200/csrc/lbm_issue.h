@@ -86,10 +86,11 @@ cudaGraphExec_t capture_graph(RunGraphs& g, Emit&& emit) {
 // step a run 7.6 us -> 6.2, three steps 14.4 -> 6.5).  Building one costs as
 // much as some 40 launches: the chunk is built for a run of at least kLongRun
 // chunks or a domain that has run before, the rest once two runs from the same
-// lattice have ended in rests of the same length (ten in a row to replace one),
-// so that a single short run pays for neither.  Where a graph cannot be built or
-// launched the steps are launched one by one, and so they are on a stream that
-// is being captured (into that graph).
+// lattice have ended in rests of the same length (to replace one, once ten in
+// a row have, none of them launched from the graph between), so that a single
+// short run pays for neither.  Where a graph cannot be built or launched the
+// steps are launched one by one, and so they are on a stream that is being
+// captured (into that graph).
 constexpr int kLongRun = 8;
 constexpr int kRestFirst = 1, kRestReplace = 9;  // equal rests before a graph
 template <class D, class Step, class Finish>
@@ -158,6 +159,7 @@ int issue_run(D* d, int n, Step&& step, Finish&& finish) {
   }
   g.ran = true;
   if (rest) {
+    g.rest_times[c0] = 0;  // the loose rests before it are no longer in a row
     if (launch(g.rest[c0], m)) return LBM_OK;
     g.drop_rest(c0);
   }

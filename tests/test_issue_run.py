@@ -1,7 +1,8 @@
 """How a run is issued (lbm_issue.h), on the host with a stand-in for the CUDA
 runtime whose calls can be made to fail: a graph that cannot be built or
 launched costs nothing but launches, a launch that is refused leaves the domain
-saying what its lattices hold and no incomplete graph behind."""
+saying what its lattices hold and no incomplete graph behind, and run lengths
+that alternate do not build a graph again and again."""
 import os
 import re
 import subprocess
@@ -54,5 +55,9 @@ def test_refused_capture_query(driver):
 def test_graphs_built(driver):
     assert driver(CREATE, 0, [6])[1] == 0
     assert driver(CREATE, 0, [6] * 5)[1] == 1
+    # lengths that alternate from one lattice, with and without a graph of one
+    assert driver(CREATE, 0, [6, 8] * 40)[1] == 0
+    assert driver(CREATE, 0, [6] * 3 + [8, 6] * 40)[1] == 1
+    assert driver(CREATE, 0, [6] * 3 + [6, 6, 8] * 40)[1] == 1
     # a new length for good: its graph takes the place of the old one
     assert driver(CREATE, 0, [6] * 3 + [8] * 30)[1] == 2
