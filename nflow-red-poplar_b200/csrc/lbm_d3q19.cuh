@@ -512,9 +512,13 @@ __host__ __device__ __forceinline__ void collide_srt_pairs(const V (&f)[Q], cons
       emit(IC<a>{}, fma_((even + odd) - f[a], inv_tau, f[a]));
       emit(IC<b>{}, fma_((even - odd) - f[b], inv_tau, f[b]));
     } else {
-      const V c = fma_(bc<V>(4.5) * eu, eu, c0);
-      emit(IC<a>{}, fma_(fma_(wr, fma_(bc<V>(3), eu, c), -f[a]), inv_tau, f[a]));
-      emit(IC<b>{}, fma_(fma_(wr, fma_(bc<V>(-3), eu, c), -f[b]), inv_tau, f[b]));
+      // feq - f with the even half against f first: what is left is of the size
+      // of the odd half, so the second rounding is an order smaller than one of
+      // feq.  (wr (c + 3 eu) - f, which rounds the sum at the size of 1 for a and
+      // b alike, left 3 to 9 % more velocity error over 100 steps.)
+      const V c = fma_(bc<V>(4.5) * eu, eu, c0), w3 = bc<V>(3) * wr;
+      emit(IC<a>{}, fma_(fma_(w3, eu, fma_(wr, c, -f[a])), inv_tau, f[a]));
+      emit(IC<b>{}, fma_(fma_(-w3, eu, fma_(wr, c, -f[b])), inv_tau, f[b]));
     }
   });
 }
