@@ -234,8 +234,9 @@ int lbm_set_solid_mask(lbm_domain* d, const unsigned char* mask) {
       d->solid = nullptr;
       return set_error(LBM_ERR_OOM, "solid mask of %lld bytes", d->N);
     }
-    if ((rc = ensure_staging(d, (size_t)d->N))) return rc;
-    unsigned char* raw = (unsigned char*)d->staging;
+    // the fields are void from here on (the domain restarts): u_x takes the
+    // caller's mask, so that no memory is needed beside the classes'
+    unsigned char* raw = (unsigned char*)d->ux;
     CK(cudaMemcpyAsync(raw, mask, (size_t)d->N, cudaMemcpyHostToDevice, d->stream));
     const dim3 b = block_of(d->g.nx);
     k_solid_class<<<grid_of(d->g, b), b, 0, d->stream>>>(d->g, raw, d->solid);
