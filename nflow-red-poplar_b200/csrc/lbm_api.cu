@@ -312,7 +312,7 @@ int lbm_import_arF(lbm_domain* d, const float* arF, int padded) {
     return set_error(LBM_ERR_NOT_FINITE, "lbm_import_arF: input holds NaN/Inf");
   }
   rc = storage_ops(d->opt.storage).import_staging(d, padded);
-  if (rc) return rc;
+  if (rc || (rc = clear_solid_planes(d, d->stream))) return rc;
   d->cur = 0;
   d->post_direct = true;
   CK(cudaMemsetAsync(d->flag + 2, 0, 2 * sizeof(int), d->stream));  // step counter

@@ -668,6 +668,17 @@ inline InitParams init_params(const lbm_domain* d) {
   return ip;
 }
 
+// No step measures a solid voxel, so beside the inlet or on the outlet the
+// boundary planes hold the zeros there that the kernel of the starting state
+// left: in the planes of even steps, and here in those of odd steps.
+inline int clear_solid_planes(lbm_domain* d, cudaStream_t st) {
+  if (!d->g.solid) return LBM_OK;
+  const size_t pb = (size_t)d->g.ny * d->g.nz * sizeof(float);
+  CK(cudaMemsetAsync(d->prho[1], 0, pb, st));
+  CK(cudaMemsetAsync(d->pu[1], 0, 6 * pb, st));
+  return LBM_OK;
+}
+
 // Launch the initial-state kernel of d on st (pull form: post lattice
 // lat[1], first collision into lat[0]; AA: arF_0 in lat[0]) and reset the
 // step state.
@@ -677,7 +688,7 @@ inline int domain_launch_init(lbm_domain* d, cudaStream_t st) {
   CK(cudaMemsetAsync(d->den[1], 0, nb, st));
   CK(cudaMemsetAsync(d->flag + 2, 0, 2 * sizeof(int), st));  // step counter
   int rc = storage_ops(d->opt.storage).launch_init(d, st);
-  if (rc) return rc;
+  if (rc || (rc = clear_solid_planes(d, st))) return rc;
   d->cur = 0;
   d->post_direct = true;
   d->aa_first = d->opt.stream_mode == LBM_STREAM_AA;
