@@ -1005,7 +1005,9 @@ __device__ __forceinline__ void aa_neighbor_face_node(const StepArgs<S>& a, int 
     const bool out = !row_in(cy(q), cz(q)) || (cx(q) == -1 && xlo) || (cx(q) == 1 && xhi);
     if constexpr (ROWS && cy(q) == 1)
       if (lid) v = aa_wall<S>(a, NODE_MOVINGWALL, v, q);
-    StoreTraits<S>::store(out ? a.dst + (opp(q) * a.qs + cell) : a.dstq[q] + cell, v, a.scale);
+    // own slots: plane opp q of the one lattice, by its pointer in the arguments
+    // (formed from a.dst and a.qs it cost registers: 36 bytes of spills, now 8)
+    StoreTraits<S>::store((out ? const_cast<S*>(a.srcq[opp(q)]) : a.dstq[q]) + cell, v, a.scale);
   });
 }
 
@@ -1076,13 +1078,22 @@ __device__ __forceinline__ void aa_step_node(const StepArgs<S>& a, int x, int y,
   });
 }
 
-// One kernel per step kind (NB = neighbor): the local step, which has no
-// box-face logic besides the open-face rules, fits 56 registers (9 CTAs of
-// 128 per SM) without spills; the neighbour step takes 72 (7 CTAs), as with
-// 64 it spills 60 bytes: 256^3 FP32 412 us a step (mean of both kinds) against
-// 422, 512x128x128 204 against 213.
+// One kernel per step kind (NB = neighbor), each with its register budget as
+// CTAs of 128 per SM.  32-bit arithmetic: the local step, which has no box-face
+// logic besides the open-face rules, fits 56 registers (9 CTAs) without spills,
+// the neighbour step 64 (8) but for a few bytes (with 72, 7 CTAs, us a step:
+// 256^3 FP32 SRT 435 against 405, MRT + LES 415 against 410; 16 FP16 64^3
+// members of a batch 107 against 98).  64-bit arithmetic holds twice the
+// registers: with the bounds above MRT + LES spilled 700 to 850 bytes; with 128
+// registers 256^3 takes 799 us, with 80 893, with those 1224; the other models
+// are best at 80 (SRT 772, at 128 789).
 template <class S, int COLL, bool LES, int NB>
-__global__ void __launch_bounds__(128, NB ? 7 : 9)
+constexpr int aa_step_ctas() {
+  if (sizeof(RealOf<S>) == 8) return COLL == COLL_MRT && LES ? 4 : 6;
+  return NB ? 8 : 9;
+}
+template <class S, int COLL, bool LES, int NB>
+__global__ void __launch_bounds__(128, aa_step_ctas<S, COLL, LES, NB>())
     k_aa_step(const __grid_constant__ StepArgs<S> a, int entry) {
   chain_wait();
   const FlatItem i = flat_item(a);
