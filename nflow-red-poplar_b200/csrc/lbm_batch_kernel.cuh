@@ -166,33 +166,37 @@ __global__ void __launch_bounds__(256, MINB) k_batch_step(const BatchTables* __r
     }
     const unsigned n0 = (t - cur.begin) * span;
     const unsigned nend = min(n0 + span, (unsigned)cur.m.nodes);
-    for (unsigned nb = n0; nb < nend; nb += 32u) {
-      const unsigned n = nb + lane;
+    auto at = [&](unsigned n, int& x, int& y, int& z) {
       const unsigned r = fastdiv(n, cur.m.mnx);
-      const int x = (int)(n - r * (unsigned)cur.m.nx);
-      const unsigned y = fastdiv(r, cur.m.mnz);
-      const int z = (int)(r - y * (unsigned)cur.m.nz);
-      // AA: one form for the warp, as in the flat kernel (with a form per lane,
-      // the face rows' for every node on a face, 20 FP32 members of 32^3 to 128^3
+      x = (int)(n - r * (unsigned)cur.m.nx);
+      y = (int)fastdiv(r, cur.m.mnz);
+      z = (int)(r - (unsigned)y * (unsigned)cur.m.nz);
+    };
+    int x, y, z;
+    if constexpr (MODE == kModeAA) {
+      // one form for the warp, as in the flat kernel (with a form per lane, the
+      // face rows' for every node on a face, 20 FP32 members of 32^3 to 128^3
       // took 544 us a step, now 447)
-      [[maybe_unused]] int faces = kFacesNone;
-      if constexpr (MODE == kModeAA) {
-        const bool row = (y == 0) | ((int)y == a.g.ny - 1) | (z == 0) | (z == a.g.nz - 1);
-        if (__any_sync(0xffffffffu, row))
+      for (unsigned nb = n0; nb < nend; nb += 32u) {
+        at(nb + lane, x, y, z);
+        int faces = kFacesNone;
+        if (__any_sync(0xffffffffu, (y == 0) | (y == a.g.ny - 1) | (z == 0) | (z == a.g.nz - 1)))
           faces = kFacesRow;
         else if (__any_sync(0xffffffffu, (x == 0) | (x == a.g.nx - 1)))
           faces = kFacesX;
+        if (nb + lane < nend)
+          aa_step_node<S, COLL, LES, false, true>(a, x, y, z, a.aa_step - 1,
+                                                  j == 0 ? cur.m.entry0 : kAAPending, faces);
       }
-      if (n >= nend) continue;
-      if constexpr (MODE == kModeAA)
-        aa_step_node<S, COLL, LES>(a, x, (int)y, z, a.aa_step - 1,
-                                   j == 0 ? cur.m.entry0 : kAAPending, faces);
-      else if constexpr (MODE == kModePaired)
-        paired_word<S, COLL, LES, false>(  // x: the word
-            a, x, (int)y, z,
-            (y == 0) | ((int)y == a.g.ny - 1) | (z == 0) | (z == a.g.nz - 1));
-      else
-        step_node<S, COLL, LES>(a, x, (int)y, z, on_face(a.g, x, (int)y, z));
+    } else {
+      for (unsigned n = n0 + lane; n < nend; n += 32u) {
+        at(n, x, y, z);
+        if constexpr (MODE == kModePaired)
+          paired_word<S, COLL, LES, false>(  // x: the word
+              a, x, y, z, (y == 0) | (y == a.g.ny - 1) | (z == 0) | (z == a.g.nz - 1));
+        else
+          step_node<S, COLL, LES>(a, x, y, z, on_face(a.g, x, y, z));
+      }
     }
   }
 }

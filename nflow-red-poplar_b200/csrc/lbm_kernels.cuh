@@ -970,8 +970,9 @@ struct AADst {
 // z face; without it only x = 0 and x = nx - 1 are looked at, which is what
 // most of the warps need that come here.  (With one form for both the 256^3
 // FP32 neighbour step took 516 us, with two 430 us.)
-// MACRO: rho and u only.
-template <class S, int COLL, bool LES, bool ROWS, bool MACRO>
+// MACRO: rho and u only.  OWN_PTR: the own slots are stored through the plane
+// pointers in the arguments, not by an address formed from a.dst and a.qs.
+template <class S, int COLL, bool LES, bool ROWS, bool MACRO, bool OWN_PTR>
 __device__ __forceinline__ void aa_neighbor_face_node(const StepArgs<S>& a, int x, int y, int z,
                                                       int cell) {
   using R = RealOf<S>;
@@ -1005,9 +1006,11 @@ __device__ __forceinline__ void aa_neighbor_face_node(const StepArgs<S>& a, int 
     const bool out = !row_in(cy(q), cz(q)) || (cx(q) == -1 && xlo) || (cx(q) == 1 && xhi);
     if constexpr (ROWS && cy(q) == 1)
       if (lid) v = aa_wall<S>(a, NODE_MOVINGWALL, v, q);
-    // own slots: plane opp q of the one lattice, by its pointer in the arguments
-    // (formed from a.dst and a.qs it cost registers: 36 bytes of spills, now 8)
-    StoreTraits<S>::store((out ? const_cast<S*>(a.srcq[opp(q)]) : a.dstq[q]) + cell, v, a.scale);
+    // own slots: plane opp q of the one lattice
+    if constexpr (OWN_PTR)
+      StoreTraits<S>::store((out ? const_cast<S*>(a.srcq[opp(q)]) : a.dstq[q]) + cell, v, a.scale);
+    else
+      StoreTraits<S>::store(out ? a.dst + (opp(q) * a.qs + cell) : a.dstq[q] + cell, v, a.scale);
   });
 }
 
@@ -1025,7 +1028,7 @@ enum { kFacesNone = 0, kFacesX = 1, kFacesRow = 2 };
 // x = nx - 1 among the warp's) or kFacesRow (nodes on a y or z face).
 // MACRO: only rho and u of arF in the layout that step would read, for a.den_out
 // and a.ux_out.
-template <class S, int COLL, bool LES, bool MACRO = false>
+template <class S, int COLL, bool LES, bool MACRO = false, bool OWN_PTR = false>
 __device__ __forceinline__ void aa_step_node(const StepArgs<S>& a, int x, int y, int z,
                                              int neighbor, int entry, int faces) {
   using R = RealOf<S>;
@@ -1034,9 +1037,9 @@ __device__ __forceinline__ void aa_step_node(const StepArgs<S>& a, int x, int y,
   const int cell = neighbor ? x + a.g.px * (z + a.g.nz * y) : cell_of(a.g, x, y, z);
   if (neighbor && faces != kFacesNone) {
     if (faces == kFacesX)
-      aa_neighbor_face_node<S, COLL, LES, false, MACRO>(a, x, y, z, cell);
+      aa_neighbor_face_node<S, COLL, LES, false, MACRO, OWN_PTR>(a, x, y, z, cell);
     else
-      aa_neighbor_face_node<S, COLL, LES, true, MACRO>(a, x, y, z, cell);
+      aa_neighbor_face_node<S, COLL, LES, true, MACRO, OWN_PTR>(a, x, y, z, cell);
     return;
   }
   R f[Q];
@@ -1090,7 +1093,17 @@ __device__ __forceinline__ void aa_step_node(const StepArgs<S>& a, int x, int y,
 template <class S, int COLL, bool LES, int NB>
 constexpr int aa_step_ctas() {
   if (sizeof(RealOf<S>) == 8) return COLL == COLL_MRT && LES ? 4 : 6;
+  if (kDev<S> && COLL == COLL_SRT && !LES) return NB ? 7 : 9;
   return NB ? 8 : 9;
+}
+// Own slots by pointer where the registers are short: FP32 MRT + LES 8 bytes of
+// spills instead of 36 (256^3 410 to 417 us a step against 436), 16-bit 2 to 12 %
+// less time; the smaller FP32 models, which spill nothing, wait longer for the
+// pointer (64^3 SRT 6.33 against 6.08).
+template <class S, int COLL, bool LES>
+constexpr bool aa_step_own_ptr() {
+  return sizeof(S) == 4 ? COLL == COLL_MRT && LES
+                        : sizeof(S) == 8 || COLL == COLL_MRT || LES;
 }
 template <class S, int COLL, bool LES, int NB>
 __global__ void __launch_bounds__(128, aa_step_ctas<S, COLL, LES, NB>())
@@ -1105,7 +1118,8 @@ __global__ void __launch_bounds__(128, aa_step_ctas<S, COLL, LES, NB>())
       faces = kFacesX;
   }
   if (!i.in) return;
-  aa_step_node<S, COLL, LES>(a, i.x, i.y, i.z, NB, entry, faces);
+  aa_step_node<S, COLL, LES, false, aa_step_own_ptr<S, COLL, LES>()>(a, i.x, i.y, i.z, NB, entry,
+                                                                     faces);
 }
 
 // rho and u of arF in the current AA layout, written through a.den_out /
