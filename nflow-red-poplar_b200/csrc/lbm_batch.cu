@@ -480,8 +480,9 @@ int issue_chunk_flat(lbm_batch* b, int steps_offered, long long* lups) {
       if (p.n == 1) {
         // one member: its single-domain kernel, launched as alone
         const lbm_domain* d = only->m->d;
-        const int nb = mode == kModeAA ? p.args[0].aa_step - 1 : 0;
-        kp.func = const_cast<void*>(t.single[model][mode][nb]);
+        const int form = mode == kModeAA ? p.args[0].aa_step - 1
+                                         : (mode == kModePull ? (int)has_struct(d->g) : 0);
+        kp.func = const_cast<void*>(t.single[model][mode][form]);
         kp.blockDim = dim3(kFlat);
         kp.gridDim = flat_grid(d->g);
         args[0] = &p.args[0];

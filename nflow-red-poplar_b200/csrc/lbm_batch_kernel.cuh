@@ -281,7 +281,8 @@ struct BatchKernels {
   BatchKernel k[4][2][kModes];
   const void* flat[4][kModes];  // k_batch_flat<S, ...>: the FlatSet<S> of the format
   // the single-domain step kernels (a set of one member, schedule 2):
-  // [model][mode][NB], NB the AA step kind (k_aa_step<.., NB>), 0 otherwise
+  // [model][mode][form], the form of an AA step its kind (k_aa_step<.., NB>), of
+  // a pull step over plain rows whether the geometry holds STRUCT nodes
   const void* single[4][kModes][2];
 };
 
@@ -304,7 +305,8 @@ const void* flat_kernel_of(int model) {
 template <class S, int COLL, bool LES>
 void set_single(BatchKernels& t, int m) {
   t.single[m][kModePull][0] = (const void*)k_step<S, COLL, LES, false>;
-  t.single[m][kModePull][1] = nullptr;
+  t.single[m][kModePull][1] =
+      kDev<S> ? t.single[m][kModePull][0] : (const void*)k_step<S, COLL, LES, false, false, !kDev<S>>;
   t.single[m][kModeAA][0] = (const void*)k_aa_step<S, COLL, LES, 0>;
   t.single[m][kModeAA][1] = (const void*)k_aa_step<S, COLL, LES, 1>;
   if constexpr (kDev<S>)

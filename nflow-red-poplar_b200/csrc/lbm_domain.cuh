@@ -374,11 +374,16 @@ cudaError_t launch_step(const lbm_domain* d, const StepArgs<S>& a, cudaStream_t 
     }
   }
   if constexpr (kDev<S>) {
-    if (a.sr) return launch_chained(k_step<S, COLL, LES, true>, gf, bf, st, a);
-  } else if ((long long)Q * d->qs * (long long)sizeof(S) <= kOnceBytes) {
-    return launch_chained(k_step<S, COLL, LES, false, true>, gf, bf, st, a);
+    return a.sr ? launch_chained(k_step<S, COLL, LES, true>, gf, bf, st, a)
+                : launch_chained(k_step<S, COLL, LES, false>, gf, bf, st, a);
+  } else {
+    const bool once = (long long)Q * d->qs * (long long)sizeof(S) <= kOnceBytes;
+    if (has_struct(d->g))
+      return once ? launch_chained(k_step<S, COLL, LES, false, true, true>, gf, bf, st, a)
+                  : launch_chained(k_step<S, COLL, LES, false, false, true>, gf, bf, st, a);
+    return once ? launch_chained(k_step<S, COLL, LES, false, true>, gf, bf, st, a)
+                : launch_chained(k_step<S, COLL, LES, false>, gf, bf, st, a);
   }
-  return launch_chained(k_step<S, COLL, LES, false>, gf, bf, st, a);
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link

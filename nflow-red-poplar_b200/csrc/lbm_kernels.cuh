@@ -450,6 +450,38 @@ __device__ __forceinline__ R initial_feq(R rd, R ux, R uy, R uz) {
   return mul_rn(mul_rn(weight<R>(q), rd), br);
 }
 
+// Boundary rules of a node whose populations with a donor outside the box hold
+// the node's own f*_{opp q}.  Only two kinds of node change the value (a fixed
+// wall keeps it): the cavity's lid (y = ny - 1 off its edges, the five
+// populations with c_y = -1), and the inlet and outlet of rows off the y and z
+// faces (x = 0, c_x = +1; x = nx - 1, c_x = -1).
+template <class S>
+__device__ __forceinline__ void face_rules(RealOf<S> (&f)[Q], const StepArgs<S>& a, int x, int y,
+                                           int z, bool face_row) {
+  const bool xlo = x == 0, xhi = x == a.g.nx - 1;
+  if (a.g.casetype == CAVITY) {
+    if (y == a.g.ny - 1 && z > 0 && z < a.g.nz - 1 && !xlo && !xhi) {
+      static_for<0, Q>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        if constexpr (cy(q) == -1) f[q] = boundary_value<S, q>(a, NODE_MOVINGWALL, f[q], y, z);
+      });
+    }
+  } else if (!face_row) {
+    if (xlo) {
+      static_for<0, Q>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        if constexpr (cx(q) == 1) f[q] = boundary_value<S, q>(a, NODE_INLET, f[q], y, z);
+      });
+    }
+    if (xhi) {
+      static_for<0, Q>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        if constexpr (cx(q) == -1) f[q] = boundary_value<S, q>(a, NODE_OUTLET, f[q], y, z);
+      });
+    }
+  }
+}
+
 // Streaming + boundaries with STRUCT nodes (kernel.cu:489-516, 659-697,
 // 566-657): a donor that is STRUCT does not stream (keStreaming skips it); a
 // FLUID node takes half-way bounce-back from its own f*_{opp q}
@@ -458,10 +490,9 @@ __device__ __forceinline__ R initial_feq(R rd, R ux, R uy, R uz) {
 // never written in the reference and keeps its initial value.  POISEUILLE,
 // and any case with a solid mask (the same rules on arbitrary voxels), for
 // the nodes of class kSolidNear: the others stream like the plain cases.  The
-// 18 mask reads per node and the initial state (a splitmix64 hash in FP64,
-// needed by the few populations without a rule) bounded the whole step while
-// every node took this path: 180x60x68 FP32 SRT + LES 53 us a step, 28 us with the
-// class byte and the initial state built only where a population needs it.
+// initial state (a splitmix64 hash in FP64) is built only where a population
+// needs it: 180x60x68 FP32 SRT + LES 53 us a step with every node on this path and
+// every state built, 28 with the class byte and the state built on demand.
 template <class S, class Addr>
 __device__ __forceinline__ void pull_struct(RealOf<S> (&f)[Q], const StepArgs<S>& a, const Addr& ad,
                                             int x, int y, int z) {
@@ -498,35 +529,62 @@ __device__ __forceinline__ void pull_struct(RealOf<S> (&f)[Q], const StepArgs<S>
   }
 }
 
-// Boundary rules of a node whose populations with a donor outside the box hold
-// the node's own f*_{opp q}.  Only two kinds of node change the value (a fixed
-// wall keeps it): the cavity's lid (y = ny - 1 off its edges, the five
-// populations with c_y = -1), and the inlet and outlet of rows off the y and z
-// faces (x = 0, c_x = +1; x = nx - 1, c_x = -1).
-template <class S>
-__device__ __forceinline__ void face_rules(RealOf<S> (&f)[Q], const StepArgs<S>& a, int x, int y,
-                                           int z, bool face_row) {
-  const bool xlo = x == 0, xhi = x == a.g.nx - 1;
-  if (a.g.casetype == CAVITY) {
-    if (y == a.g.ny - 1 && z > 0 && z < a.g.nz - 1 && !xlo && !xhi) {
+// The same for the step kernel of such geometries: donor or own population by
+// address, so that the 19 loads go out together, and the rules after them.  us a
+// step FP32 MRT + LES: channel 96x64x64 with 15 % of the voxels solid at random,
+// where nearly every node is beside one, 36.2 -> 26.3 (33.5 while every node took
+// the path above), 256x200x180 835 -> 477 (806); 180x60x68 with two spheres 23.3 ->
+// 21.9.  It takes 64 registers where the path above fits 56, so the kernels that
+// step plain members beside (batches) keep that one, and so do the 16-bit steps,
+// which the path above had not slowed.
+template <class S, class Addr>
+__device__ __forceinline__ void pull_struct_select(RealOf<S> (&f)[Q], const StepArgs<S>& a, const Addr& ad,
+                                            int x, int y, int z) {
+  using R = RealOf<S>;
+  const int t = node_type(a.g, x, y, z);
+  const bool pipe = a.g.casetype == POISEUILLE;
+  const long long n = x + (long long)a.g.nx * (z + (long long)a.g.nz * y);
+  unsigned in = 0u, solid = 0u;  // donors inside the box; those that are STRUCT
+  static_for<0, Q>([&](auto qc) {
+    constexpr int q = decltype(qc)::value;
+    const int xs = x - cx(q), ys = y - cy(q), zs = z - cz(q);
+    const bool inside = (unsigned)xs < (unsigned)a.g.nx && (unsigned)ys < (unsigned)a.g.ny &&
+                        (unsigned)zs < (unsigned)a.g.nz;
+    bool s = pipe && (ys - 25) * (ys - 25) + (zs - 25) * (zs - 25) > 400;
+    if (a.g.solid && inside)
+      s |= a.g.solid[n - (cx(q) + a.g.nx * (cz(q) + (long long)a.g.nz * cy(q)))] == kSolidStruct;
+    if (inside) in |= 1u << q;
+    if (inside && s) solid |= 1u << q;
+  });
+  // two words instead of 19 conditions held until their loads: 56 to 64
+  // registers, 64 to 79 without
+  asm("" : "+r"(in), "+r"(solid));
+  const unsigned donor = in & ~solid, out = ~in & ((1u << Q) - 1);
+  unsigned keep = t != NODE_FLUID ? solid : 0u;  // populations that keep their initial value
+  static_for<0, Q>([&](auto qc) {
+    constexpr int q = decltype(qc)::value;
+    f[q] = ld(donor >> q & 1u ? ad.donor(q) : ad.own(opp(q)), q, ad.inv_scale());
+  });
+  if (!pipe) {
+    face_rules<S>(f, a, x, y, z, (y == 0) | (y == a.g.ny - 1) | (z == 0) | (z == a.g.nz - 1));
+  } else if (t == NODE_INLET || t == NODE_OUTLET) {
+    if (out)
       static_for<0, Q>([&](auto qc) {
         constexpr int q = decltype(qc)::value;
-        if constexpr (cy(q) == -1) f[q] = boundary_value<S, q>(a, NODE_MOVINGWALL, f[q], y, z);
+        if (out >> q & 1u) f[q] = boundary_value<S, q>(a, t, f[q], y, z);
       });
-    }
-  } else if (!face_row) {
-    if (xlo) {
-      static_for<0, Q>([&](auto qc) {
-        constexpr int q = decltype(qc)::value;
-        if constexpr (cx(q) == 1) f[q] = boundary_value<S, q>(a, NODE_INLET, f[q], y, z);
-      });
-    }
-    if (xhi) {
-      static_for<0, Q>([&](auto qc) {
-        constexpr int q = decltype(qc)::value;
-        if constexpr (cx(q) == -1) f[q] = boundary_value<S, q>(a, NODE_OUTLET, f[q], y, z);
-      });
-    }
+  } else {
+    keep |= out;
+  }
+  if (keep) {
+    const InitState is = initial_state(a.g, a.init_kind, a.seed, a.noise_amp, (float)a.rho0,
+                                       (float)a.ulx, (float)a.uly, (float)a.ulz, a.inlet_u, x, y,
+                                       z, t);
+    static_for<0, Q>([&](auto qc) {
+      constexpr int q = decltype(qc)::value;
+      if (keep >> q & 1u)
+        f[q] = to_internal<S, q>(initial_feq<R, q>(R(is.den), R(is.ux), R(is.uy), R(is.uz)));
+    });
   }
 }
 
@@ -538,11 +596,15 @@ __device__ __forceinline__ void face_rules(RealOf<S> (&f)[Q], const StepArgs<S>&
 // warp that holds one, so that the warp does not run both.  (When each lane
 // took its own form, with the rules of every node type inlined 18 times, a
 // 16^3 FP32 step took 3.8 us, 64^3 9.3 us and 96^3 27.3 us; now 2.1, 6.7 and 22.4.)
-template <class S, bool ONCE = false, class Addr>
+// STRUCT: the kernel is that of the geometries with STRUCT nodes.
+template <class S, bool ONCE = false, bool STRUCT = false, class Addr>
 __device__ __forceinline__ void pull(RealOf<S> (&f)[Q], const StepArgs<S>& a, const Addr& ad, int x,
                                      int y, int z, bool faces) {
   if (has_struct(a.g) && struct_class(a.g, x, y, z) != kSolidFree) {
-    pull_struct<S>(f, a, ad, x, y, z);
+    if constexpr (STRUCT)
+      pull_struct_select<S>(f, a, ad, x, y, z);
+    else
+      pull_struct<S>(f, a, ad, x, y, z);
   } else if (!faces) {
     static_for<0, Q>([&](auto qc) {
       constexpr int q = decltype(qc)::value;
@@ -706,7 +768,8 @@ __device__ __forceinline__ void finish_node(const RealOf<S> (&f)[Q], const StepA
 // LES, collision, store.  Shared by the single-domain and batched kernels,
 // so a domain gets the same bits alone and in a batch (only where the
 // arguments are held differs, not the arithmetic).
-template <class S, int COLL, bool LES, bool SR = false, bool ONCE = false, class Addr>
+template <class S, int COLL, bool LES, bool SR = false, bool ONCE = false, bool STRUCT = false,
+          class Addr>
 __device__ __forceinline__ void step_node_at(const StepArgs<S>& a, const Addr& ad, int x, int y,
                                              int z, bool faces) {
   using R = RealOf<S>;
@@ -714,7 +777,7 @@ __device__ __forceinline__ void step_node_at(const StepArgs<S>& a, const Addr& a
   // 323, 362, 464, 495, 1105)
   if (has_struct(a.g) && struct_class(a.g, x, y, z) == kSolidStruct) return;
   R f[Q];
-  pull<S, ONCE>(f, a, ad, x, y, z, faces);
+  pull<S, ONCE, STRUCT>(f, a, ad, x, y, z, faces);
   finish_node<S, COLL, LES, SR>(f, a, ad, x, y, z);
 }
 
@@ -732,16 +795,30 @@ __device__ __forceinline__ void step_node(const StepArgs<S>& a, int x, int y, in
   step_node_at<S, COLL, LES>(a, PlaneAddr<S>(a, x + a.g.px * (z + a.g.nz * y)), x, y, z, faces);
 }
 
-// The fused step.  grid = flat_grid, one thread per node.
-template <class S, int COLL, bool LES, bool SR = false, bool ONCE = false>
-__global__ void __launch_bounds__(128) k_step(const __grid_constant__ StepArgs<S> a) {
+// The fused step.  grid = flat_grid, one thread per node.  STRUCT: for geometries
+// with STRUCT nodes, a kernel of its own so that the registers of
+// pull_struct_select do not bound the others (64^3 FP32 SRT 6.09 us a step, 6.18
+// with it in theirs).  CTAs per SM are left to the compiler (0) but for two with
+// STRUCT nodes: FP64 MRT + LES, where 96 registers are better than the 106 it takes
+// (channel 180x120x128 with a sphere 147 us a step against 163), and FP32 SRT +
+// LES, where 64 without spills are better than 64 with (180x120x128 84.1 against
+// 84.5 side by side; the other FP32 models lose 2 to 8 % by a bound).
+template <class S, int COLL, bool LES, bool STRUCT>
+constexpr int step_ctas() {
+  if (!STRUCT || !LES) return 0;
+  if (sizeof(RealOf<S>) == 8) return COLL == COLL_MRT ? 5 : 0;
+  return COLL == COLL_SRT ? 8 : 0;
+}
+template <class S, int COLL, bool LES, bool SR = false, bool ONCE = false, bool STRUCT = false>
+__global__ void __launch_bounds__(128, step_ctas<S, COLL, LES, STRUCT>())
+    k_step(const __grid_constant__ StepArgs<S> a) {
   chain_wait();
   bump_step_counter<SR>(a);
   const FlatItem i = flat_item(a);
   const bool faces = __any_sync(0xffffffffu, i.face_row | (i.x == 0) | (i.x == a.g.nx - 1));
   if (!i.in) return;
-  step_node_at<S, COLL, LES, SR, ONCE>(a, PlaneAddr<S>(a, i.x + a.g.px * (i.z + a.g.nz * i.y)), i.x,
-                                       i.y, i.z, faces);
+  step_node_at<S, COLL, LES, SR, ONCE, STRUCT>(
+      a, PlaneAddr<S>(a, i.x + a.g.px * (i.z + a.g.nz * i.y)), i.x, i.y, i.z, faces);
 }
 
 // ------------------------------------------------------------------ //
@@ -1084,12 +1161,12 @@ __device__ __forceinline__ void aa_step_node(const StepArgs<S>& a, int x, int y,
 // One kernel per step kind (NB = neighbor), each with its register budget as
 // CTAs of 128 per SM.  32-bit arithmetic: the local step, which has no box-face
 // logic besides the open-face rules, fits 56 registers (9 CTAs) without spills,
-// the neighbour step 64 (8) but for a few bytes (with 72, 7 CTAs, us a step:
-// 256^3 FP32 SRT 435 against 405, MRT + LES 415 against 410; 16 FP16 64^3
-// members of a batch 107 against 98).  64-bit arithmetic holds twice the
-// registers: with the bounds above MRT + LES spilled 700 to 850 bytes; with 128
-// registers 256^3 takes 799 us, with 80 893, with those 1224; the other models
-// are best at 80 (SRT 772, at 128 789).
+// the neighbour step 64 (8) but for a few bytes; with 72 (7 CTAs) 256^3 FP32 SRT
+// takes 435 us a step against 405, 16 FP16 64^3 members of a batch 107 against 98.
+// (16-bit SRT is the exception: 49x48x48 4.67 with 72, 4.87 with 64.)  64-bit
+// arithmetic holds twice the registers: with the bounds of FP32 MRT + LES spilled
+// 700 to 850 bytes; with 128 registers 256^3 takes 799 us, with 80 893, with those
+// 1224; the other models are best at 80 (SRT 772, at 128 789).
 template <class S, int COLL, bool LES, int NB>
 constexpr int aa_step_ctas() {
   if (sizeof(RealOf<S>) == 8) return COLL == COLL_MRT && LES ? 4 : 6;
