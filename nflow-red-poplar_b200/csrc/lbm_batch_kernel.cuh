@@ -306,7 +306,8 @@ template <class S, int COLL, bool LES>
 void set_single(BatchKernels& t, int m) {
   t.single[m][kModePull][0] = (const void*)k_step<S, COLL, LES, false>;
   t.single[m][kModePull][1] =
-      kDev<S> ? t.single[m][kModePull][0] : (const void*)k_step<S, COLL, LES, false, false, !kDev<S>>;
+      kDev<S> ? t.single[m][kModePull][0]
+              : (const void*)k_step<S, COLL, LES, false, false, !kDev<S>>;
   t.single[m][kModeAA][0] = (const void*)k_aa_step<S, COLL, LES, 0>;
   t.single[m][kModeAA][1] = (const void*)k_aa_step<S, COLL, LES, 1>;
   if constexpr (kDev<S>)

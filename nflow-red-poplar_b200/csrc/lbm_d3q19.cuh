@@ -369,33 +369,30 @@ __host__ __device__ __forceinline__ void make_pairs(const V (&f)[Q], PairState<V
     const V g = ps.d[8] - ps.d[7], h = ps.d[3] + ps.d[4];
     ps.jz = (g - h) - ps.d[1];
     ps.nm18 = g + h;
-    return;
-  }
-  // rho = f0 + sum s; j_alpha = sum_p c_alpha(a_p) d_p
-  V acc = ps.s[0] + ps.s[1];
-  acc = acc + ps.s[2];
-  V diag = ps.s[3] + ps.s[4];
-  diag = diag + ps.s[5];
-  diag = diag + ps.s[6];
-  diag = diag + ps.s[7];
-  diag = diag + ps.s[8];
-  ps.rho = ps.f0 + (acc + diag);
-  if constexpr (DEV)
+  } else {
+    // rho = f0 + sum s; j_alpha = sum_p c_alpha(a_p) d_p
+    V acc = ps.s[0] + ps.s[1];
+    acc = acc + ps.s[2];
+    V diag = ps.s[3] + ps.s[4];
+    diag = diag + ps.s[5];
+    diag = diag + ps.s[6];
+    diag = diag + ps.s[7];
+    diag = diag + ps.s[8];
+    ps.rho = ps.f0 + (acc + diag);
     ps.rho_full = ps.rho + bc<V>(1);
-  else
-    ps.rho_full = ps.rho;
-  V jx = ps.d[0] + ps.d[3];
-  jx = jx - ps.d[4];
-  jx = jx + ps.d[5];
-  ps.jx = jx - ps.d[6];
-  V jy = ps.d[2] + ps.d[5];
-  jy = jy + ps.d[6];
-  jy = jy + ps.d[7];
-  ps.jy = jy + ps.d[8];
-  V jz = ps.d[8] - ps.d[1];
-  jz = jz - ps.d[3];
-  jz = jz - ps.d[4];
-  ps.jz = jz - ps.d[7];
+    V jx = ps.d[0] + ps.d[3];
+    jx = jx - ps.d[4];
+    jx = jx + ps.d[5];
+    ps.jx = jx - ps.d[6];
+    V jy = ps.d[2] + ps.d[5];
+    jy = jy + ps.d[6];
+    jy = jy + ps.d[7];
+    ps.jy = jy + ps.d[8];
+    V jz = ps.d[8] - ps.d[1];
+    jz = jz - ps.d[3];
+    jz = jz - ps.d[4];
+    ps.jz = jz - ps.d[7];
+  }
 }
 
 // Smagorinsky tau_eddy from the pair sums (same closed form as les_tau_eddy)
@@ -421,38 +418,39 @@ __host__ __device__ __forceinline__ V les_tau_eddy_pairs(const PairState<V>& ps,
     qq = fma_(bc<V>(2), off, qq);
     return fma_(bc<V>(0.5), vsqrt(fma_(tau, tau, (les_c * vsqrt(qq)) * inv_rho)),
                 bc<V>(-0.5) * tau);
+  } else {
+    V pxx = s[0] + s[3];
+    pxx = pxx + s[4];
+    pxx = pxx + s[5];
+    pxx = pxx + s[6];
+    V pyy = s[2] + s[5];
+    pyy = pyy + s[6];
+    pyy = pyy + s[7];
+    pyy = pyy + s[8];
+    V pzz = s[1] + s[3];
+    pzz = pzz + s[4];
+    pzz = pzz + s[7];
+    pzz = pzz + s[8];
+    const V pxy = s[5] - s[6];  // f11 - f12 - f13 + f14
+    const V pxz = s[4] - s[3];  // -f7 + f8 + f9 - f10
+    const V pyz = s[8] - s[7];  // -f15 + f16 + f17 - f18
+    const V r3 = ps.rho * bc<V>(1.0 / 3.0);
+    const V txx = pxx - fma_(ps.jx, ux, r3);
+    const V tyy = pyy - fma_(ps.jy, uy, r3);
+    const V tzz = pzz - fma_(ps.jz, uz, r3);
+    const V txy = pxy - ps.jx * uy;
+    const V txz = pxz - ps.jx * uz;
+    const V tyz = pyz - ps.jy * uz;
+    V off = txy * txy;
+    off = fma_(txz, txz, off);
+    off = fma_(tyz, tyz, off);
+    V qq = txx * txx;
+    qq = fma_(tyy, tyy, qq);
+    qq = fma_(tzz, tzz, qq);
+    qq = fma_(bc<V>(2), off, qq);
+    return fma_(bc<V>(0.5), vsqrt(fma_(tau, tau, (les_c * vsqrt(qq)) * inv_rho)),
+                bc<V>(-0.5) * tau);
   }
-  V pxx = s[0] + s[3];
-  pxx = pxx + s[4];
-  pxx = pxx + s[5];
-  pxx = pxx + s[6];
-  V pyy = s[2] + s[5];
-  pyy = pyy + s[6];
-  pyy = pyy + s[7];
-  pyy = pyy + s[8];
-  V pzz = s[1] + s[3];
-  pzz = pzz + s[4];
-  pzz = pzz + s[7];
-  pzz = pzz + s[8];
-  const V pxy = s[5] - s[6];  // f11 - f12 - f13 + f14
-  const V pxz = s[4] - s[3];  // -f7 + f8 + f9 - f10
-  const V pyz = s[8] - s[7];  // -f15 + f16 + f17 - f18
-  const V r3 = ps.rho * bc<V>(1.0 / 3.0);
-  const V txx = pxx - fma_(ps.jx, ux, r3);
-  const V tyy = pyy - fma_(ps.jy, uy, r3);
-  const V tzz = pzz - fma_(ps.jz, uz, r3);
-  const V txy = pxy - ps.jx * uy;
-  const V txz = pxz - ps.jx * uz;
-  const V tyz = pyz - ps.jy * uz;
-  V off = txy * txy;
-  off = fma_(txz, txz, off);
-  off = fma_(tyz, tyz, off);
-  V qq = txx * txx;
-  qq = fma_(tyy, tyy, qq);
-  qq = fma_(tzz, tzz, qq);
-  qq = fma_(bc<V>(2), off, qq);
-  return fma_(bc<V>(0.5), vsqrt(fma_(tau, tau, (les_c * vsqrt(qq)) * inv_rho)),
-              bc<V>(-0.5) * tau);
 }
 
 // SRT in pair form: feq_a, feq_abar share w rho (1 - 1.5u^2 + 4.5 (c.u)^2)
@@ -500,22 +498,24 @@ __host__ __device__ __forceinline__ void collide_srt_pairs(const V (&f)[Q], cons
       else eu = acc_term<cz(a)>(eu, uz);
     }
     const V wr = wclass(a) == 1 ? wr1 : wr2;
-    V even;
-    if constexpr (DEV)
-      even = bc<V>(wclass(a) == 1 ? 1.0 / 18.0 : 1.0 / 36.0) *
-             fma_(rho, fma_(bc<V>(4.5) * eu, eu, c0), ps.rho);
-    else
-      even = wr * fma_(bc<V>(4.5) * eu, eu, c0);
-    const V odd = (bc<V>(3) * wr) * eu;
+    auto even = [&] {
+      if constexpr (DEV)
+        return bc<V>(wclass(a) == 1 ? 1.0 / 18.0 : 1.0 / 36.0) *
+               fma_(rho, fma_(bc<V>(4.5) * eu, eu, c0), ps.rho);
+      else
+        return wr * fma_(bc<V>(4.5) * eu, eu, c0);
+    };
+    auto odd = [&] { return (bc<V>(3) * wr) * eu; };
     if constexpr (FROM_PAIRS) {
       // s* = s + (2 even - s) inv,  d* = d + (2 odd - d) inv
-      const V ss = fma_(fma_(bc<V>(2), even, -ps.s[p]), inv_tau, ps.s[p]);
-      const V dd = fma_(fma_(bc<V>(2), odd, -ps.d[p]), inv_tau, ps.d[p]);
+      const V ss = fma_(fma_(bc<V>(2), even(), -ps.s[p]), inv_tau, ps.s[p]);
+      const V dd = fma_(fma_(bc<V>(2), odd(), -ps.d[p]), inv_tau, ps.d[p]);
       emit(IC<a>{}, bc<V>(0.5) * (ss + dd));
       emit(IC<b>{}, bc<V>(0.5) * (ss - dd));
     } else if constexpr (DEV) {
-      emit(IC<a>{}, fma_((even + odd) - f[a], inv_tau, f[a]));
-      emit(IC<b>{}, fma_((even - odd) - f[b], inv_tau, f[b]));
+      const V ev = even(), od = odd();
+      emit(IC<a>{}, fma_((ev + od) - f[a], inv_tau, f[a]));
+      emit(IC<b>{}, fma_((ev - od) - f[b], inv_tau, f[b]));
     } else {
       // feq - f with the even half against f first: what is left is of the size
       // of the odd half, so the second rounding is an order smaller than one of
@@ -530,8 +530,8 @@ __host__ __device__ __forceinline__ void collide_srt_pairs(const V (&f)[Q], cons
 }
 
 // The same collision for populations f, with the conserved parts of the
-// moments cancelled by hand and every multiply-add explicit, so that the
-// scalar and the packed kernels round alike whatever the compiler would fuse:
+// moments cancelled by hand and every multiply-add explicit, so that kernels
+// round alike whatever the compiler would fuse:
 //   m1 - meq1 = 19 (B - f0 - j.j/rho0)          (M_1 f + 11 rho = 19 (B - f0))
 //   m4 - meq4 = 5/3 jx - 5 d0, likewise 6 and 8
 // About 150 additions, multiplications and fused pairs with the pair sums,
@@ -628,18 +628,14 @@ __host__ __device__ __forceinline__ void collide_mrt_fused(const V (&f)[Q], cons
 // formed from s/d, relaxation dm'_k = s_k (m_k - meq_k) / |row_k|^2, back
 // transform f_a -= E_p + O_p, f_abar -= E_p - O_p (or, FROM_PAIRS, the same
 // rebuilt from s - 2E and d - 2O).  emit(q, value) receives the results.
-// DEV: f, s, d hold deviations g = f - w and ps.rho = rho - 1; every
+// The form for deviations (DEV): f, s, d hold g = f - w and ps.rho = rho - 1; every
 // equilibrium moment but meq_2 is then the same expression in ps.rho (the
 // rest state's moments M w are (1, -11, 3, 0, ...) and meq_1 = -11 rho + ...
 // is linear in rho), meq_2 adds the constant p.e2c.
-template <bool FROM_PAIRS, class V, class R, bool DEV = false, class Emit>
-__host__ __device__ __forceinline__ void collide_mrt_pairs(const V (&f)[Q], const PairState<V>& ps,
+template <bool FROM_PAIRS, class V, class R, class Emit>
+__host__ __device__ __forceinline__ void collide_mrt_dev(const V (&f)[Q], const PairState<V>& ps,
                                                            V s_nu, const MrtParams<R>& p,
                                                            Emit&& emit) {
-  if constexpr (!DEV) {
-    collide_mrt_fused<FROM_PAIRS, V, R>(f, ps, s_nu, p, emit);
-    return;
-  }
   const V* s = ps.s;
   const V* d = ps.d;
   const V rho = ps.rho, jx = ps.jx, jy = ps.jy, jz = ps.jz;
@@ -677,14 +673,9 @@ __host__ __device__ __forceinline__ void collide_mrt_pairs(const V (&f)[Q], cons
   const V meq11 = rho0_inv * (jyy - jzz);
   // ---- relaxed, pre-scaled differences dm'_k = s_k (m_k - meq_k)/|row|^2 ----
   const V e1 = bc<V>(1.19 / 2394.0) * (m1 - fma_(bc<V>(19), jj0, bc<V>(-11) * rho));
-  V e2;
-  if constexpr (DEV)
-    e2 = bc<V>(1.4 / 252.0) *
-         ((m2 - fma_(bcast_param<V>(p.wepsj), jj0, bcast_param<V>(p.weps) * rho)) +
-          bcast_param<V>(p.e2c));
-  else
-    e2 = bc<V>(1.4 / 252.0) *
-         (m2 - fma_(bcast_param<V>(p.wepsj), jj0, bcast_param<V>(p.weps) * rho));
+  const V e2 = bc<V>(1.4 / 252.0) *
+               ((m2 - fma_(bcast_param<V>(p.wepsj), jj0, bcast_param<V>(p.weps) * rho)) +
+                bcast_param<V>(p.e2c));
   const V e4 = bc<V>(1.2 / 40.0) * fma_(bc<V>(2.0 / 3.0), jx, m4);
   const V e6 = bc<V>(1.2 / 40.0) * fma_(bc<V>(2.0 / 3.0), jy, m6);
   const V e8 = bc<V>(1.2 / 40.0) * fma_(bc<V>(2.0 / 3.0), jz, m8);
@@ -741,6 +732,16 @@ __host__ __device__ __forceinline__ void collide_mrt_pairs(const V (&f)[Q], cons
       emit(IC<b>{}, f[b] - (E[q] - O[q]));
     }
   });
+}
+
+template <bool FROM_PAIRS, class V, class R, bool DEV = false, class Emit>
+__host__ __device__ __forceinline__ void collide_mrt_pairs(const V (&f)[Q], const PairState<V>& ps,
+                                                           V s_nu, const MrtParams<R>& p,
+                                                           Emit&& emit) {
+  if constexpr (DEV)
+    collide_mrt_dev<FROM_PAIRS, V, R>(f, ps, s_nu, p, emit);
+  else
+    collide_mrt_fused<FROM_PAIRS, V, R>(f, ps, s_nu, p, emit);
 }
 
 }  // namespace lbm

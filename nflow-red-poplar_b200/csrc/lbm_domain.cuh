@@ -521,8 +521,8 @@ inline void free_all(lbm_domain* d) {
 
 
 // Row layout of a single domain (d->in, d->opt and d->g's sizes and mask are
-// set): 16-bit pull (A/B) domains use paired rows where the paired step applies (no
-// STRUCT nodes, nx >= 11), 16-bit AA domains quad rows where they fit, unless
+// set): 16-bit pull (A/B) domains use paired rows where the paired step applies
+// (paired_kernel_applies), 16-bit AA domains quad rows where they fit, unless
 // another kernel is asked for.
 inline int domain_rows(const lbm_domain* d) {
   const lbm_options& o = d->opt;

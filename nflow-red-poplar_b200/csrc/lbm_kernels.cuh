@@ -248,12 +248,10 @@ struct FlatItem {
 // with the planes that the step before wrote last, which are still in the 126
 // MB L2 (forwards, a lattice larger than L2 evicts each plane before its next
 // use).  Up to kTurnBytes(AA) of lattices: beyond, what is left in the L2 is a few
-// per cent of a step, and domains stepped side by side lose that and 1 % more.  us a step forwards -> alternating: FP32 in place 112^3 35.9 -> 28.8,
-// 128^3 55 -> 46, 160^3 105 -> 96, 256^3 413 -> 408; FP32 pull 128^3 51.7 -> 50.3;
-// FP64 pull 80^3 26.4 -> 22.6, 256^3 765 -> 756; FP16 pull 160^3 79 -> 74; FP16 in
-// place 160^3 68 -> 61.  (Fetching the source of a pull step with an evict-first
-// policy helps while one lattice fits the L2, 96^3 FP32 21.3 -> 19.1, and costs 4 %
-// above, where the other half of a split sector is gone before its use.)
+// per cent of a step, and domains stepped side by side lose that and 1 % more.
+// us a step forwards -> alternating: FP32 in place 112^3 35.9 -> 28.8, 128^3 55 ->
+// 46, 160^3 105 -> 96; FP32 pull 128^3 51.7 -> 50.3; FP64 pull 80^3 26.4 -> 22.6;
+// FP16 pull 160^3 79 -> 74; FP16 in place 160^3 68 -> 61.
 template <class S>
 __device__ __forceinline__ FlatItem flat_item(const StepArgs<S>& a) {
   const unsigned bx = a.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
@@ -538,8 +536,8 @@ __device__ __forceinline__ void pull_struct(RealOf<S> (&f)[Q], const StepArgs<S>
 // step plain members beside (batches) keep that one, and so do the 16-bit steps,
 // which the path above had not slowed.
 template <class S, class Addr>
-__device__ __forceinline__ void pull_struct_select(RealOf<S> (&f)[Q], const StepArgs<S>& a, const Addr& ad,
-                                            int x, int y, int z) {
+__device__ __forceinline__ void pull_struct_select(RealOf<S> (&f)[Q], const StepArgs<S>& a,
+                                                   const Addr& ad, int x, int y, int z) {
   using R = RealOf<S>;
   const int t = node_type(a.g, x, y, z);
   const bool pipe = a.g.casetype == POISEUILLE;
@@ -926,7 +924,7 @@ __global__ void __launch_bounds__(128)
 }
 
 // ------------------------------------------------------------------ //
-// AA streaming (in place, one lattice), for the cavity geometry.
+// AA streaming (in place, one lattice), for the cavity and the channel.
 //
 // Two layouts alternate.  "Natural": slot (x, q) holds the post-stream,
 // post-boundary f_q(x) (arF).  A local step reads its node's natural
@@ -948,8 +946,8 @@ __global__ void __launch_bounds__(128)
 // export kernels), with the face buffers of that step.  The natural layout
 // is "complete" after the initial state and an import (every slot holds
 // arF, rules applied) and "pending" after a neighbour step.  Same node
-// arithmetic as the pull step; the two kernels agree to within a few FP32
-// roundings (the compiler may fuse a multiply-add differently in each).
+// arithmetic as the pull step: in FP32 and 16-bit storage, built without
+// multiply-add contraction, the same bits.
 //
 // Face buffers: AA step k reads arF_{k-1} and writes its rho / u into
 // prho[k & 1] / pu[k & 1] (make_args with k); the rules for arF_{k-1} read
@@ -1445,9 +1443,9 @@ __device__ __forceinline__ uint32_t pack_pair_sr<__nv_bfloat16>(F2 v, float scal
   return d;
 }
 
-// the paired step kernel applies to the domain (else: plain rows); nx >= 11
-// keeps both x faces out of each other's words and every hi lane's x + 1
-// donor of a real node inside the row
+// the paired step kernel applies to the domain (else: plain rows): px / 2 <= nx -
+// 2 (nx of 6 to 8, 10 and more) keeps both x faces out of each other's words and
+// every hi lane's x + 1 donor of a real node inside the row
 __host__ __device__ __forceinline__ bool paired_kernel_applies(const Geometry& g) {
   return !has_struct(g) && (g.px >> 1) <= g.nx - 2;
 }
