@@ -946,8 +946,8 @@ __global__ void __launch_bounds__(128)
 // export kernels), with the face buffers of that step.  The natural layout
 // is "complete" after the initial state and an import (every slot holds
 // arF, rules applied) and "pending" after a neighbour step.  Same node
-// arithmetic as the pull step: in FP32 and 16-bit storage, built without
-// multiply-add contraction, the same bits.
+// arithmetic as the pull step: in FP32, built without multiply-add contraction,
+// the same bits.
 //
 // Face buffers: AA step k reads arF_{k-1} and writes its rho / u into
 // prho[k & 1] / pu[k & 1] (make_args with k); the rules for arF_{k-1} read
