@@ -473,11 +473,6 @@ __host__ __device__ __forceinline__ void collide_srt_pairs(const V (&f)[Q], cons
     emit(IC<0>{}, fma_(bc<V>(1.0 / 3.0) * fma_(rho, c0, ps.rho) - ps.f0, inv_tau, ps.f0));
   else
     emit(IC<0>{}, fma_(fma_(rho * bc<V>(1.0 / 3.0), c0, -ps.f0), inv_tau, ps.f0));
-  if constexpr (!DEV && !FROM_PAIRS) {
-    ux = bc<V>(3) * ux;
-    uy = bc<V>(3) * uy;
-    uz = bc<V>(3) * uz;
-  }
   const V wr1 = rho * bc<V>(1.0 / 18.0), wr2 = rho * bc<V>(1.0 / 36.0);
   static_for<0, 9>([&](auto pc) {
     constexpr int p = decltype(pc)::value;
@@ -520,11 +515,11 @@ __host__ __device__ __forceinline__ void collide_srt_pairs(const V (&f)[Q], cons
       // feq - f with the even half against f first: what is left is of the size
       // of the odd half, so the second rounding is an order smaller than one of
       // feq.  (wr (c + 3 eu) - f, which rounds the sum at the size of 1 for a and
-      // b alike, left 3 to 9 % more velocity error over 100 steps.)  eu holds
-      // 3 c.u here.
-      const V c = fma_(bc<V>(0.5) * eu, eu, c0);
-      emit(IC<a>{}, fma_(fma_(wr, eu, fma_(wr, c, -f[a])), inv_tau, f[a]));
-      emit(IC<b>{}, fma_(fma_(-wr, eu, fma_(wr, c, -f[b])), inv_tau, f[b]));
+      // b alike, left 3 to 9 % more velocity error over 100 steps; so does 3 u
+      // rounded first, by a third of that.)
+      const V c = fma_(bc<V>(4.5) * eu, eu, c0), w3 = bc<V>(3) * wr;
+      emit(IC<a>{}, fma_(fma_(w3, eu, fma_(wr, c, -f[a])), inv_tau, f[a]));
+      emit(IC<b>{}, fma_(fma_(-w3, eu, fma_(wr, c, -f[b])), inv_tau, f[b]));
     }
   });
 }
